@@ -2469,7 +2469,7 @@ int conv_pair_capacity() {
 }
 
 int encode_tiled_f16(CUtensorMap* map, const void* ptr, int rank, const unsigned long long* dims,
-                     const unsigned long long* strides_bytes, const unsigned* box, bool swizzle128) {
+                     const unsigned long long* strides_bytes, const unsigned* box, int swizzle_bytes) {
     if (!g_encode_tiled || rank < 1 || rank > 5) return FVM_ERR_SETUP;
     cuuint64_t d[5], st[4];
     cuuint32_t b[5], es[5];
@@ -2481,7 +2481,10 @@ int encode_tiled_f16(CUtensorMap* map, const void* ptr, int rank, const unsigned
     }
     const CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, static_cast<cuuint32_t>(rank), const_cast<void*>(ptr),
                                       d, st, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                      swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                                      swizzle_bytes == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                      : swizzle_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                      : swizzle_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                                            : CU_TENSOR_MAP_SWIZZLE_NONE,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? FVM_OK : FVM_ERR_TMAP;
 }
@@ -2683,6 +2686,27 @@ int stem_s2_launch(const void* x, const void* w, const void* bias, void* y, int 
     return launch_conv_kernel(tmap_a, tmap_b, tmap_y, tmap_y, p, grid, smem, stream);
 }
 
+// Whether a gated 1x1 convolution over one image (M pixels) runs on conv_split_kernel: CTAs per tile (0: no) and the tile
+// width. Both estimates (us) are fits to CUDA-graph timings on B200: the per-image-weights mode takes 6.3 us for one k-block and
+// 8.6 for 18 (EfficientNet-B0, one image); the split kernel's launch with its epilogue, the k-blocks one CTA streams, the rows it
+// finishes and the exchange add up to 4.7 us for 672 -> 112 at 14x14 (four CTAs per tile) and 4.3 for 1152 -> 192 at 7x7.
+// Only one wave of CTAs counts: with two per SM both slow down.
+static int split_rule(int M, int K, int kblocks, const DeviceState* st, int* bn) {
+    const int mt = (M + BM - 1) / BM, w = K <= 32 ? 32 : 64;
+    const double rows = M < BM ? static_cast<double>(M) / BM : 1.0;
+    double best = 0.95 * (6.0 + 0.22 * kblocks);
+    int split = 0;
+    for (int s = 1; s <= 8 && s <= kblocks && static_cast<long long>(mt) * ((K + w - 1) / w) * s <= st->sms; ++s) {
+        const double t = 3.5 + 0.22 * ((kblocks + s - 1) / s) + 2.3 * rows / s + 0.05 * s;
+        if (t < best) {
+            best = t;
+            split = s;
+            *bn = w;
+        }
+    }
+    return split;
+}
+
 int conv2d_launch(const void* x, const void* w, const void* bias, const void* res, const float* scale, void* y, int N,
                   int H, int W, int C, int K, int R, int S, int ph, int pw, int sh, int sw, int dh, int dw,
                   long long ldx, long long ldy, long long ldr, int act, int force_bn, int ph_hi, int pw_hi,
@@ -2695,13 +2719,19 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
     if (!x || !w || !y) return FVM_ERR_ARG;
     // force_bn: low 16 bits = output-channel tile (0 = choose), bits 16..23 = sub-tiles per tile (0 = choose),
     // bits 24..25 = weight-resident mode (0 = choose, 1 = on, 2 = off), bits 26..27 = halo mode, bits 28..29 = stream-K
-    // (same coding), bit 30 = CTA pairs (conv_pair_kernel) on
+    // (same coding; 3 = conv_split_kernel with the CTAs per tile in bits 16..23), bit 30 = CTA pairs (conv_pair_kernel) on
     int force_pair = force_bn > 0 ? ((force_bn >> 30) & 1) : 0;
     const bool free_choice = force_bn <= 0;
-    const int force_sk = force_bn > 0 ? ((force_bn >> 28) & 3) : 0;
-    const int force_halo = force_bn > 0 ? ((force_bn >> 26) & 3) : 0;
+    int force_sk = force_bn > 0 ? ((force_bn >> 28) & 3) : 0;
+    int force_halo = force_bn > 0 ? ((force_bn >> 26) & 3) : 0;
     const int force_bres = force_bn > 0 ? ((force_bn >> 24) & 3) : 0;
-    const int force_mt = force_bn > 0 ? ((force_bn >> 16) & 0xff) : 0;
+    int force_mt = force_bn > 0 ? ((force_bn >> 16) & 0xff) : 0;
+    int split = 0, wdyn = 0;        // conv_split_kernel: CTAs per tile (0: not used); weights not constant
+    if (force_sk == 3) {
+        split = force_mt;
+        if (split <= 0 || force_pair || force_halo == 1 || force_bres == 1 || gsg > 0) return FVM_ERR_ARG;
+        force_sk = force_mt = 0;
+    }
     force_bn = force_bn > 0 ? (force_bn & 0xffff) : 0;
     if (N <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0 || R <= 0 || S <= 0) return FVM_ERR_ARG;
     if ((C & 7) || (K & 7) || (ldx & 7) || (ldy & 7) || (res && (ldr & 7))) return FVM_ERR_ARG;
@@ -2717,6 +2747,18 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
     if (P <= 0 || Q <= 0) return FVM_ERR_ARG;
     const long long M_ll = static_cast<long long>(N) * P * Q;
     if (M_ll > 0x7fffff00ll) return FVM_ERR_ARG;
+
+    // One image's weights are an ordinary weight tensor, except that the preceding kernel has written it: where the cluster
+    // kernel is faster it takes them. (Convolutions with constant weights get there by the host's per-layer timing.)
+    if (free_choice && w_per_image && N == 1) split = split_rule(static_cast<int>(M_ll), K, (C + BK - 1) / BK, st, &force_bn);
+    if (split > 0) {
+        force_halo = 2;
+        if (w_per_image && N == 1 && R == 1 && S == 1 && sh == 1 && sw == 1 && !ph && !pw && !ph_hi && !pw_hi) {
+            w_per_image = 0;
+            wdyn = 1;
+        }
+        if (w_per_image) return FVM_ERR_ARG;
+    }
 
     ConvParams p;
     memset(&p, 0, sizeof(p));
@@ -2759,7 +2801,7 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
         const int Kp16 = (K + 31) / 32 * 32;   // tiles are multiples of 32 channels
         SmemPlan tp;
         const int tpk = (C == 8 || C == 16) ? BK / C : 1;      // taps per k-block in tap-packed mode
-        p.tapk = (!gsg && (C == 8 || C == 16) && R * S > 1 && Kp16 <= 256 && (force_bn <= 0 || force_bn >= Kp16) &&
+        p.tapk = (!gsg && !split && (C == 8 || C == 16) && R * S > 1 && Kp16 <= 256 && (force_bn <= 0 || force_bn >= Kp16) &&
                   plan_smem(Kp16, 1, (R * S + tpk - 1) / tpk, K, true, false, &tp)) ? C : 0;
         if (p.tapk) {
             p.kblocks = (R * S + tpk - 1) / tpk;
@@ -2793,9 +2835,12 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
     // 28x28 and smaller maps of a ResNet at batch 64; measured there: 10-25 % faster than the best single-CTA tile).
     // Tile width from the same measurements: all of K (up to 256) for deep reductions without a residual, else 128.
     static const int auto_pairs = [] { const char* v = getenv("FVM_B200_PAIR"); return (v && v[0] == '0') ? 0 : 1; }();
-    if (free_choice && auto_pairs && !gsg && !p.tapk && !p.halo && !p.wb && st->pair_clusters > 0 && C >= 24 && K >= 64 &&
+    if (free_choice && auto_pairs && !split && !gsg && !p.tapk && !p.halo && !p.wb && st->pair_clusters > 0 && C >= 24 && K >= 64 &&
         p.m_tiles <= 4 * st->sms) {
-        const int bn = (K <= 128 || (K <= 256 && !res && p.kblocks >= 8)) ? (K + 31) / 32 * 32 : 128;
+        int bn = (K <= 128 || (K <= 256 && !res && p.kblocks >= 8)) ? (K + 31) / 32 * 32 : 128;
+        // tiles for less than half of the pairs: 64 channels wide, so that twice as many SMs share the weights (one image,
+        // 1x1 256 -> 1024 at 14x14 5.2 -> 4.5 us, 128 -> 512 at 28x28 4.9 -> 4.2)
+        if (K > 64 && static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((K + bn - 1) / bn) * 2 <= st->pair_clusters) bn = 64;
         SmemPlan tp;
         if (plan_smem(bn, 1, p.kblocks, K, false, false, &tp, 0, true)) {
             force_pair = 1;
@@ -2874,7 +2919,7 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
     }
     SmemPlan sp;
     p.bres = 0;
-    if (!p.sk && !p.wb && !p.tapk && !p.pair && force_bres != 2 && p.n_tiles <= st->sms) {
+    if (!split && !p.sk && !p.wb && !p.tapk && !p.pair && force_bres != 2 && p.n_tiles <= st->sms) {
         const long long wbytes = static_cast<long long>(p.kblocks) * p.BN * BK * 2;
         const int cta_per_n = st->sms / p.n_tiles;
         const bool worth = p.m_tiles >= 2 * cta_per_n;
@@ -2945,10 +2990,10 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
                                             static_cast<unsigned long long>(N)};
         const unsigned box[3] = {64, BM, 1};
         const unsigned long long ystr[2] = {static_cast<unsigned long long>(ldy) * 2, static_cast<unsigned long long>(P) * Q * ldy * 2};
-        if (encode_tiled_f16(&tmap_y, y, 3, dims, ystr, box, true) != FVM_OK) return FVM_ERR_TMAP;
+        if (encode_tiled_f16(&tmap_y, y, 3, dims, ystr, box, 128) != FVM_OK) return FVM_ERR_TMAP;
         if (res) {
             const unsigned long long rstr[2] = {static_cast<unsigned long long>(ldr) * 2, static_cast<unsigned long long>(P) * Q * ldr * 2};
-            if (encode_tiled_f16(&tmap_r, res, 3, dims, rstr, box, true) != FVM_OK) return FVM_ERR_TMAP;
+            if (encode_tiled_f16(&tmap_r, res, 3, dims, rstr, box, 128) != FVM_OK) return FVM_ERR_TMAP;
         } else {
             tmap_r = tmap_y;
         }
@@ -3004,7 +3049,7 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
                                             static_cast<unsigned long long>(N)};
         const unsigned long long strides[2] = {static_cast<unsigned long long>(ldx) * 2, static_cast<unsigned long long>(P) * Q * ldx * 2};
         const unsigned box[3] = {BK, static_cast<unsigned>(p.a_rows), 1};
-        if (encode_tiled_f16(&tmap_a, x, 3, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+        if (encode_tiled_f16(&tmap_a, x, 3, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
     } else if (!p.im2col) {
         cuuint64_t dims[2] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(p.M)};
         cuuint64_t strides[1] = {static_cast<cuuint64_t>(ldx) * 2};
@@ -3042,6 +3087,27 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
             reinterpret_cast<uint64_t*>(&tmap_a)[1] &= ~(1ull << 21);
     }
 
+    if (split > 0) {
+        SplitParams q;
+        memset(&q, 0, sizeof(q));
+        q.M = p.M; q.K = K; q.P = P; q.Q = Q; q.S = S;
+        q.sh = sh; q.sw = sw; q.ph = ph; q.pw = pw; q.dh = dh; q.dw = dw;
+        q.cchunks = p.cchunks; q.kblocks = p.kblocks; q.im2col = p.im2col;
+        q.BN = p.BN; q.n_tiles = p.n_tiles; q.split = split;
+        q.act = act;
+        q.wdyn = wdyn;
+        q.bias = p.bias;
+        q.res = static_cast<const __half*>(res);
+        q.scale = scale;
+        q.y = static_cast<__half*>(y);
+        q.ldy = ldy; q.ldr = ldr;
+        q.div_split = fastdiv_init(static_cast<uint32_t>(split));
+        q.div_ntiles = p.div_ntiles; q.div_pq = p.div_pq; q.div_q = p.div_q;
+        q.status = p.status;
+        size_t split_smem = 0;
+        if (!conv_split_plan(&q, &split_smem) || static_cast<long long>(p.m_tiles) * p.n_tiles * split > 0x7fffffffll) return FVM_ERR_ARG;
+        return conv_split_launch(tmap_a, tmap_b, q, split_smem, stream);
+    }
     const long long total_tiles = static_cast<long long>(p.m_tiles) * p.n_tiles;
     int grid = static_cast<int>(total_tiles < st->sms ? total_tiles : st->sms);
     if (p.bres) {
@@ -3196,7 +3262,7 @@ int conv_chain_launch(const fvm_chain_layer* layers, int n, cudaStream_t stream)
             const unsigned long long dims[2] = {static_cast<unsigned long long>(a.K), static_cast<unsigned long long>(L.M)};
             const unsigned long long strides[1] = {static_cast<unsigned long long>(a.ldr) * 2};
             const unsigned box[2] = {64, BM};
-            if (encode_tiled_f16(&cp.ext_res[n_ext], a.res, 2, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+            if (encode_tiled_f16(&cp.ext_res[n_ext], a.res, 2, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
             L.res_ext = n_ext++;
         }
         for (int j = 0; j < i; ++j) {
@@ -3240,7 +3306,7 @@ int conv_chain_launch(const fvm_chain_layer* layers, int n, cudaStream_t stream)
             const unsigned long long dims[2] = {static_cast<unsigned long long>(a.K), static_cast<unsigned long long>(L.M)};
             const unsigned long long strides[1] = {static_cast<unsigned long long>(a.ldy) * 2};
             const unsigned box[2] = {64, BM};
-            if (encode_tiled_f16(&L.tmap_y, a.y, 2, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+            if (encode_tiled_f16(&L.tmap_y, a.y, 2, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
         }
         {   // weights [K][R*S][C]: this CTA's half of an n-tile per load
             const unsigned long long dims[3] = {static_cast<unsigned long long>(a.C), static_cast<unsigned long long>(a.R) * a.S,
@@ -3248,13 +3314,13 @@ int conv_chain_launch(const fvm_chain_layer* layers, int n, cudaStream_t stream)
             const unsigned long long strides[2] = {static_cast<unsigned long long>(a.C) * 2,
                                                    static_cast<unsigned long long>(a.R) * a.S * a.C * 2};
             const unsigned box[3] = {BK, 1, static_cast<unsigned>(L.BN / 2)};
-            if (encode_tiled_f16(&L.tmap_b, a.w, 3, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+            if (encode_tiled_f16(&L.tmap_b, a.w, 3, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
         }
         if (!L.im2col) {
             const unsigned long long dims[2] = {static_cast<unsigned long long>(a.C), static_cast<unsigned long long>(L.M)};
             const unsigned long long strides[1] = {static_cast<unsigned long long>(a.ldx) * 2};
             const unsigned box[2] = {BK, BM};
-            if (encode_tiled_f16(&L.tmap_a, a.x, 2, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+            if (encode_tiled_f16(&L.tmap_a, a.x, 2, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
         } else {
             const int up_w = a.pw - (a.S - 1) * a.dw, up_h = a.ph - (a.R - 1) * a.dh;
             if (a.pw > 127 || a.ph > 127 || up_w < -128 || up_h < -128 || (a.S - 1) * a.dw > 255 || (a.R - 1) * a.dh > 255)
@@ -3373,16 +3439,16 @@ int conv_dual_launch(const void* x, const void* w1, const void* b1, const void* 
         const unsigned long long dims[2] = {static_cast<unsigned long long>(C1), Mu};
         const unsigned long long strides[1] = {static_cast<unsigned long long>(ldx) * 2};
         const unsigned box[2] = {BK, BM};
-        if (encode_tiled_f16(&tmap_a, x, 2, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+        if (encode_tiled_f16(&tmap_a, x, 2, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
     }
     {
         const unsigned long long dims[2] = {static_cast<unsigned long long>(K1), Mu};
         const unsigned long long ystr[1] = {static_cast<unsigned long long>(ldy) * 2};
         const unsigned box[2] = {64, BM};
-        if (encode_tiled_f16(&tmap_y, y, 2, dims, ystr, box, true) != FVM_OK) return FVM_ERR_TMAP;
+        if (encode_tiled_f16(&tmap_y, y, 2, dims, ystr, box, 128) != FVM_OK) return FVM_ERR_TMAP;
         if (res) {
             const unsigned long long rstr[1] = {static_cast<unsigned long long>(ldr) * 2};
-            if (encode_tiled_f16(&tmap_r, res, 2, dims, rstr, box, true) != FVM_OK) return FVM_ERR_TMAP;
+            if (encode_tiled_f16(&tmap_r, res, 2, dims, rstr, box, 128) != FVM_OK) return FVM_ERR_TMAP;
         } else {
             tmap_r = tmap_y;
         }
@@ -3391,19 +3457,19 @@ int conv_dual_launch(const void* x, const void* w1, const void* b1, const void* 
         const unsigned long long dims[2] = {static_cast<unsigned long long>(K2), Mu};
         const unsigned long long zstr[1] = {static_cast<unsigned long long>(ldz) * 2};
         const unsigned box[2] = {64, BM};
-        if (encode_tiled_f16(&tmap_z, z, 2, dims, zstr, box, true) != FVM_OK) return FVM_ERR_TMAP;
+        if (encode_tiled_f16(&tmap_z, z, 2, dims, zstr, box, 128) != FVM_OK) return FVM_ERR_TMAP;
     }
     {
         const unsigned long long dims[3] = {static_cast<unsigned long long>(C1), 1ull, static_cast<unsigned long long>(K1)};
         const unsigned long long strides[2] = {static_cast<unsigned long long>(C1) * 2, static_cast<unsigned long long>(C1) * 2};
         const unsigned box[3] = {BK, 1, 128};
-        if (encode_tiled_f16(&tmap_w1, w1, 3, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+        if (encode_tiled_f16(&tmap_w1, w1, 3, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
     }
     {
         const unsigned long long dims[3] = {static_cast<unsigned long long>(K1), 1ull, static_cast<unsigned long long>(K2)};
         const unsigned long long strides[2] = {static_cast<unsigned long long>(K1) * 2, static_cast<unsigned long long>(K1) * 2};
         const unsigned box[3] = {BK, 1, static_cast<unsigned>(K2)};
-        if (encode_tiled_f16(&tmap_w2, w2, 3, dims, strides, box, true) != FVM_OK) return FVM_ERR_TMAP;
+        if (encode_tiled_f16(&tmap_w2, w2, 3, dims, strides, box, 128) != FVM_OK) return FVM_ERR_TMAP;
     }
     const int grid = p.m_tiles < st->sms ? p.m_tiles : st->sms;
     cudaLaunchConfig_t cfg;

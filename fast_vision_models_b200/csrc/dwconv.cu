@@ -401,7 +401,7 @@ extern "C" int fvm_dwconv_f16(const void* x, const void* w_rsc, const void* bias
                                                static_cast<unsigned long long>(H) * W * ldx * 2};
         const unsigned box[4] = {static_cast<unsigned>(p.cbv * 8), static_cast<unsigned>(p.tile_w),
                                  static_cast<unsigned>(p.tile_h), 1u};
-        const int rc = encode_tiled_f16(&tmap, x, 4, dims, strides, box, /*swizzle128=*/false);
+        const int rc = encode_tiled_f16(&tmap, x, 4, dims, strides, box, 0);
         if (rc != FVM_OK) return rc;
     }
     const long long bx = static_cast<long long>(p.tiles_x) * p.tiles_y * p.vblocks;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/fvm_b200.h"
+#include "ptx_sm100.cuh"
 
 namespace fvm {
 
@@ -32,15 +33,34 @@ void count_launch();
 int conv_host_init();
 int conv_pair_capacity();
 // cuTensorMapEncodeTiled for an fp16 tensor of `rank` dimensions (innermost first): sizes, byte strides of dimensions
-// 1.., box; no interleave, 128-byte swizzle or none, zero fill outside the tensor. Returns an FVM_* status.
+// 1.., box; no interleave, swizzle of 128, 64 or 32 bytes or none (0), zero fill outside the tensor. Returns an FVM_* status.
 int encode_tiled_f16(CUtensorMap* map, const void* ptr, int rank, const unsigned long long* dims,
-                     const unsigned long long* strides_bytes, const unsigned* box, bool swizzle128);
+                     const unsigned long long* strides_bytes, const unsigned* box, int swizzle_bytes);
 int stem_s2_launch(const void* x, const void* w, const void* bias, void* y, int N, int H, int W, int K, int R, int S,
                    int ph, int pw, long long ldy, int act, cudaStream_t stream);
 int conv2d_launch(const void* x, const void* w, const void* bias, const void* res, const float* scale, void* y, int N,
                   int H, int W, int C, int K, int R, int S, int ph, int pw, int sh, int sw, int dh, int dw,
                   long long ldx, long long ldy, long long ldr, int act, int force_bn, int ph_hi, int pw_hi,
                   cudaStream_t stream, int w_per_image = 0, int gsg = 0, int gsk = 0);
+// Cluster split-K convolution (conv_split.cu): one 128 x BN output tile per cluster of `split` CTAs.
+struct SplitParams {
+    int M, K, P, Q, S, sh, sw, ph, pw, dh, dw;
+    int cchunks, kblocks, im2col;
+    int BN, n_tiles, split;
+    int lg_bn, stages, tmem_cols;      // from conv_split_plan
+    uint32_t red_bytes;
+    int act;
+    int wdyn;                          // weights written by the preceding kernel: fetched after the wait for it
+    const __half* bias;
+    const __half* res;
+    const float* scale;
+    __half* y;
+    long long ldy, ldr;
+    FastDiv div_split, div_ntiles, div_pq, div_q;
+    int* status;
+};
+bool conv_split_plan(SplitParams* p, size_t* smem);
+int conv_split_launch(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b, const SplitParams& p, size_t smem, cudaStream_t stream);
 int conv_chain_launch(const fvm_chain_layer* layers, int n, cudaStream_t stream);
 int conv_dual_launch(const void* x, const void* w1, const void* b1, const void* res, void* y, const void* w2, const void* b2,
                      void* z, long long M, int C1, int K1, int K2, long long ldx, long long ldr, long long ldy, long long ldz,

@@ -203,6 +203,13 @@ class FusedConv(nn.Module):
         if self.w.shape[1] > 16 and ops.query(4) > 0:
             # CTA pairs (bit 30): two SMs share each tile of 256 pixels and each fetches half of the weight tile; same bits
             cands += [c | (1 << 30) for c in widths]
+        if self.w.shape[1] > 16 and rows <= 148 * 128:
+            # few tiles: one tile per cluster with the reduction split over its CTAs (bits 28..29 = 3, CTAs in bits 16..23),
+            # where all CTAs run at once
+            kblocks = R_ * S_ * ((self.w.shape[1] + 63) // 64)
+            for c in (64, 128):
+                tiles = ((rows + 127) // 128) * ((K + c - 1) // c)
+                cands += [(3 << 28) | (n << 16) | c for n in (2, 3, 4, 6, 8) if n <= kblocks and tiles * n <= 148]
         best = 0
         if len(cands) > 1:
             # Candidates are timed in rounds (every candidate once per round, best burst kept), so that a drift of the

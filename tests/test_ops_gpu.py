@@ -282,6 +282,39 @@ def test_conv_cta_pairs_are_refused_where_they_do_not_apply():
         ops.conv_fused(x, w, None, None, (1, 1), (1, 1), 0, tile_n=(1 << 30) | (2 << 16))      # with two sub-tiles
 
 
+@pytest.mark.parametrize("case", [
+    # N, H, W, C, K, R, pad, stride, dil, res, scale, act, bn, split
+    (1, 7, 7, 512, 512, 3, 1, 1, 1, False, False, 1, 64, 8),        # 49 of 128 rows, slices of 7 rows (the last has none to do)
+    (1, 14, 14, 256, 256, 3, 1, 2, 1, True, False, 1, 64, 7),       # uneven runs of k-blocks, residual
+    (3, 13, 17, 72, 136, 3, 2, 1, 2, True, True, 5, 128, 6),        # dilation, ragged channels, tiles over images, fp32 scale
+    (1, 1, 1, 2048, 1000, 1, 0, 1, 1, False, False, 0, 64, 8),      # one row
+    (2, 1, 1, 2048, 1000, 1, 0, 1, 1, False, False, 2, 128, 5),     # two rows for five CTAs
+    (1, 12, 11, 24, 24, 1, 0, 1, 1, True, False, 3, 32, 1),         # a single k-block, 24 of 32 columns, a second tile of 4 rows
+    (2, 16, 16, 320, 200, 1, 0, 1, 1, True, False, 6, 128, 2),      # 64 rows per CTA: the most units per thread
+])
+def test_conv_split_matches_oracle(case):
+    # one tile per cluster, the reduction split over its CTAs: against the oracle, and the same bits twice in a row (the
+    # partial sums are added in the order of the CTAs). Also the per-image weight form with one image where it applies.
+    N, H, W, C, K, Rr, pad, stride, dil, res, scale, act, bn, split = case
+    x, w, b = gen((N, C, H, W), 71), gen((K, C, Rr, Rr), 72, 0.02), gen((K,), 73, 0.1)
+    P = (H + 2 * pad - dil * (Rr - 1) - 1) // stride + 1
+    Q = (W + 2 * pad - dil * (Rr - 1) - 1) // stride + 1
+    r = gen((N, K, P, Q), 74) if res else None
+    sc = torch.rand(K, generator=torch.Generator().manual_seed(75)) + 0.5 if scale else None
+    ref = R.conv_fused_ref(x, w, b, r, (pad, pad), (stride, stride), act, (dil, dil), sc)
+    code = (3 << 28) | (split << 16) | bn
+    args = (cl(x), cl(w), b.to(DEV), None if r is None else cl(r), (pad, pad), (stride, stride), act)
+    kw = dict(dilation=(dil, dil), scale=None if sc is None else sc.to(DEV), tile_n=code)
+    y = ops.conv_fused(*args, **kw)
+    assert ops.last_status() == 0
+    close(y, ref)
+    assert torch.equal(y, ops.conv_fused(*args, **kw))
+    if N == 1 and Rr == 1 and K % 8 == 0:
+        yw = ops.conv1x1_wbatch(args[0], cl(w).reshape(1, K, C).contiguous(), args[2], args[3], act)
+        assert ops.last_status() == 0
+        close(yw, ref)
+
+
 def _resnet_stage(N, H, W, cin, mid, blocks, stride, seed):
     """Weights and a runner for a ResNet bottleneck stage (torchvision layout: the stride sits on the 3x3 convolution
     and on the 1x1 downsample of the first block). run() returns every layer's output, in launch order."""
