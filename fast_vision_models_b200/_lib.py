@@ -25,7 +25,7 @@ CSRC = os.path.join(_HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(_HERE), "include")
 LIB_NAME = "libfvm_b200.so"
 LIB_PATH = os.path.join(_HERE, LIB_NAME)          # the in-tree location
-SOURCES = ["abi.cu", "conv_tcgen05.cu", "conv_split.cu", "bandwidth.cu", "dwconv.cu"]
+SOURCES = ["abi.cu", "conv_tcgen05.cu", "conv_split.cu", "bandwidth.cu", "dwconv.cu", "dwconv_mma.cu"]
 HEADERS = ["fvm_internal.h", "ptx_sm100.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared"]

@@ -6,8 +6,8 @@
 // zero fill, the SM spends no instruction on addresses or bounds of the input, and every input byte crosses L2 -> SM
 // about once. Several small CTAs share an SM, so one CTA's copy is in flight while others compute.
 //
-//   dw_tile_kernel<S, SW, ACT>   square 3/5/7-tap filters, stride 1 or 2, no dilation (every depthwise layer of
-//                                EfficientNet and ConvNeXt). Thread = 8 channels x 8 consecutive output columns of one
+//   dw_tile_kernel<S, SW, ACT>   square 3/5-tap filters, stride 1 or 2, and 7-tap filters with stride 2, no dilation (every
+//                                depthwise layer of EfficientNet; 7x7 stride 1 is in dwconv_mma.cu). Thread = 8 channels x 8 consecutive output columns of one
 //                                output row; one kernel row of weights and the 64 accumulators live in registers.
 //                                Arithmetic of the reference's dwconv2 (classification/fast/csrc/r3.cu:354-415, its
 //                                default mode): fp16x2 FMAs within a kernel row starting from zero, fp32 across rows,
@@ -318,7 +318,7 @@ static bool dw_plan(int N, int H, int W, int C, int R, int S, int ph, int pw, in
     p.act = act;
     p.ldy = ldy;
     const int cv = C >> 3;
-    out->tile_kernel = R == S && (S == 3 || S == 5 || S == 7) && dh == 1 && dw == 1 && sh == sw && (sw == 1 || sw == 2);
+    out->tile_kernel = R == S && (S == 3 || S == 5 || (S == 7 && sw == 2)) && dh == 1 && dw == 1 && sh == sw && (sw == 1 || sw == 2);
     // Candidates: channel blocks from the widest acceptable one down, cell grids px x py with px a power of two. Among
     // the candidates whose product of (useful lanes) x (useful cells: tiles overhang the map) is within 15 % of the best,
     // the one with the least staged bytes per output pixel (least border) is taken. Measured on B200: small CTAs win
@@ -360,6 +360,11 @@ static bool dw_plan(int N, int H, int W, int C, int R, int S, int ph, int pw, in
     return true;
 }
 
+// 7x7 stride-1 filters without dilation have a tensor-core form (dwconv_mma.cu).
+static bool dw_on_tensor_cores(int N, int H, int W, int C, int R, int S, int ph, int pw, int sh, int sw, int dh, int dw) {
+    return R == 7 && S == 7 && sh == 1 && sw == 1 && dh == 1 && dw == 1 && dw_mma_runs(N, H, W, C, ph, pw);
+}
+
 }  // namespace fvm
 
 using namespace fvm;
@@ -369,6 +374,7 @@ extern "C" int fvm_dwconv_pool_slots(int N, int H, int W, int C, int R, int S, i
     DwPlan plan;
     if (N <= 0 || H <= 0 || W <= 0 || C <= 0 || (C & 7) || R <= 0 || S <= 0 || sh <= 0 || sw <= 0 || dh <= 0 || dw <= 0 || ph < 0 || pw < 0)
         return -1;
+    if (dw_on_tensor_cores(N, H, W, C, R, S, ph, pw, sh, sw, dh, dw)) return dw_mma_slots(N, H, W, C, ph, pw);
     if (!dw_plan(N, H, W, C, R, S, ph, pw, sh, sw, dh, dw, C, 0, &plan)) return -1;
     return plan.p.tiles_x * plan.p.tiles_y;
 }
@@ -386,6 +392,8 @@ extern "C" int fvm_dwconv_f16(const void* x, const void* w_rsc, const void* bias
         return FVM_ERR_ARG;
     DeviceState* st = device_state();
     if (!st) return FVM_ERR_SETUP;
+    if (dw_on_tensor_cores(N, H, W, C, R, S, ph, pw, sh, sw, dh, dw))
+        return dw_mma_launch(x, w_rsc, bias, y, pool_partial, N, H, W, C, ph, pw, ldx, ldy, act, static_cast<cudaStream_t>(stream));
     DwPlan plan;
     if (!dw_plan(N, H, W, C, R, S, ph, pw, sh, sw, dh, dw, ldy, act, &plan)) return FVM_ERR_ARG;
     DwParams& p = plan.p;
@@ -429,7 +437,7 @@ extern "C" int fvm_dwconv_f16(const void* x, const void* w_rsc, const void* bias
     if (plan.tile_kernel) {
         if (S == 3) { if (sw == 1) DW_ACT(3, 1); else DW_ACT(3, 2); }
         else if (S == 5) { if (sw == 1) DW_ACT(5, 1); else DW_ACT(5, 2); }
-        else { if (sw == 1) DW_ACT(7, 1); else DW_ACT(7, 2); }
+        else DW_ACT(7, 2);
     } else {
         DW_LAUNCH(dw_any_kernel);
     }

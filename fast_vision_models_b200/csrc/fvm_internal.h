@@ -61,6 +61,12 @@ struct SplitParams {
 };
 bool conv_split_plan(SplitParams* p, size_t* smem);
 int conv_split_launch(const CUtensorMap& tmap_a, const CUtensorMap& tmap_b, const SplitParams& p, size_t smem, cudaStream_t stream);
+// Stride-1 7x7 depthwise convolution on the tensor cores (dwconv_mma.cu): whether a layer runs there, its squeeze slots, its
+// launch.
+bool dw_mma_runs(int N, int H, int W, int C, int ph, int pw);
+int dw_mma_slots(int N, int H, int W, int C, int ph, int pw);
+int dw_mma_launch(const void* x, const void* w, const void* bias, void* y, float* pool_partial, int N, int H, int W, int C,
+                  int ph, int pw, long long ldx, long long ldy, int act, cudaStream_t stream);
 int conv_chain_launch(const fvm_chain_layer* layers, int n, cudaStream_t stream);
 int conv_dual_launch(const void* x, const void* w1, const void* b1, const void* res, void* y, const void* w2, const void* b2,
                      void* z, long long M, int C1, int K1, int K2, long long ldx, long long ldr, long long ldy, long long ldz,

@@ -825,6 +825,43 @@ def test_dwconv_any_shape_matches_oracle(case):
     close(y, ref)
 
 
+@pytest.mark.parametrize("case", [
+    # N, H, W, C, ph, pw, act, bias: 7x7 stride 1 on the tensor cores; strips of 8 columns, 16 per tile
+    (1, 1, 1, 8, 3, 3, 0, True),            # one output
+    (2, 8, 8, 16, 3, 3, 0, False),          # one strip per image row
+    (5, 7, 9, 24, 3, 3, 3, True),           # two strips, the second one column wide; several images per tile, a ragged last tile
+    (17, 7, 7, 40, 3, 3, 0, True),          # more images than strips
+    (1, 61, 59, 8, 3, 3, 1, True),          # rows and columns past the last segment
+    (2, 30, 200, 16, 0, 6, 5, True),        # wide: more than 16 strips per row, uneven padding
+    (3, 13, 6, 8, 3, 0, 0, True),           # no column padding: no output column but the first
+])
+def test_dwconv_7x7_on_tensor_cores(case):
+    N, H, W, C, ph, pw, act, bias = case
+    if W + 2 * pw < 7:
+        W = 7
+    x, w, b = gen((N, C, H, W), 81), gen((7, 7, C), 82, 0.1), gen((C,), 83, 0.1)
+    ref = R.dwconv_ref(x, w, b if bias else None, (1, 1), (ph, pw), act, (1, 1))
+    y, partial = ops.dwconv(cl(x), w.to(DEV), b.to(DEV) if bias else None, (1, 1), (ph, pw), act, pool=True)
+    assert ops.last_status() == 0
+    close(y, ref)
+    # squeeze sums of the rounded outputs: fp32 sums of at most 200 x 30 values in another order
+    sums = y.float().sum((2, 3)).cpu()
+    assert (partial.sum(1).cpu() - sums).abs().max() <= 1e-5 * y.float().abs().sum((2, 3)).max().cpu() + 1e-5
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan"), -float("inf")])
+def test_dwconv_7x7_non_finite_values_stay_in_their_windows(bad):
+    # the zeros of the Toeplitz matrices must not meet an infinity or a NaN: exactly the outputs whose window holds it change
+    x, w = gen((2, 8, 20, 20), 84), gen((7, 7, 8), 85, 0.1)
+    clean = ops.dwconv(cl(x), w.to(DEV), None, (1, 1), (3, 3), 0)
+    x[1, 5, 9, 11] = bad
+    y = ops.dwconv(cl(x), w.to(DEV), None, (1, 1), (3, 3), 0)
+    hit = torch.zeros(2, 8, 20, 20, dtype=torch.bool)
+    hit[1, 5, 6:13, 8:15] = True
+    assert not torch.isfinite(y.cpu()[hit]).any()
+    close(y.cpu()[~hit], clean.cpu()[~hit])
+
+
 @pytest.mark.parametrize("case", [(3, 144, 19, 19, 3, 1, 3), (2, 96, 30, 30, 7, 1, 0), (2, 336, 17, 23, 5, 2, 3),
                                   (2, 48, 40, 40, 3, 1, 3), (2, 64, 12, 12, 3, 1, 1)])
 def test_dwconv_fused_squeeze_is_exact_and_deterministic(case):
