@@ -18,6 +18,13 @@ union V8 {
 __device__ __forceinline__ uint4 ldg16(const __half* p) { return __ldg(reinterpret_cast<const uint4*>(p)); }
 __device__ __forceinline__ void stg16(__half* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
 
+// An activation that the preceding kernel wrote, in a kernel that may start before that one has ended (programmatic dependent
+// launch): an ordinary load, which pdl_wait orders; the read-only path (ld.global.nc) is for data no running kernel writes.
+__device__ __forceinline__ uint4 ld16(const __half* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ void to_f8(const uint4& u, float (&f)[8]) {
     V8 v;
     v.u = u;
@@ -165,6 +172,8 @@ static constexpr int GAP_VX = 32, GAP_RY = 8;
 __global__ void gap_partial_kernel(const __half* __restrict__ x, float* __restrict__ partial, int HW, int C,
                                    long long ldx, int splits, int chunk, __half* __restrict__ y_direct, float inv_hw) {
     __shared__ float red[GAP_RY][GAP_VX][8];
+    pdl_wait();
+    pdl_trigger();
     const int cv = C >> 3;
     const int v = blockIdx.x * GAP_VX + threadIdx.x;
     const int split = blockIdx.y;
@@ -176,7 +185,7 @@ __global__ void gap_partial_kernel(const __half* __restrict__ x, float* __restri
         const __half* base = x + n * HW * ldx + v * 8;
         for (int px = p0 + threadIdx.y; px < p1; px += GAP_RY) {
             float f[8];
-            to_f8(ldg16(base + px * ldx), f);
+            to_f8(ld16(base + px * ldx), f);
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[j] += f[j];
         }
@@ -197,12 +206,14 @@ __global__ void gap_partial_kernel(const __half* __restrict__ x, float* __restri
 
 __global__ void gap_final_kernel(const float* __restrict__ partial, __half* __restrict__ y, int C, int splits,
                                  float inv_hw, long long total) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const long long n = i / C;
     const int c = static_cast<int>(i - n * C);
     float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += partial[(n * splits + k) * C + c];
+    for (int k = 0; k < splits; ++k) s += __ldcg(partial + (n * splits + k) * C + c);
     y[i] = __float2half_rn(s * inv_hw);
 }
 
@@ -218,54 +229,66 @@ static int gap_splits(int N, int HW, int C, int sms) {
 }
 
 // ------------------------------------------------------------------------------------------- squeeze-excite gate
-// gridDim.y blocks per image: each computes h = half(act(W1 g + b1)) (warp per output, lanes stride over C; the
-// squeeze FC is small, so it is recomputed per block rather than exchanged) and its slice of s = half(W2 h + b2)
-// (thread per output). Rounding points follow the two conv_fused calls the reference issues on [N,C,1,1] tensors.
-__global__ void se_gate_kernel(const void* __restrict__ g_in, const __half* __restrict__ w1,
-                               const __half* __restrict__ b1, const __half* __restrict__ w2,
-                               const __half* __restrict__ b2, __half* __restrict__ s_out, int C, int Cs, int act,
-                               float mean_scale, int slots, int sgroups) {
+// A cluster of CTAs per image, CTA r owns `per` channels: their squeeze means, their part of h = half(act(W1 g + b1)) (all Cs
+// rows over the own channels), and their outputs of s = half(W2 h + b2). The partial rows are exchanged through distributed
+// shared memory and added in rank order, so every weight is read once per image (blocks that each computed all of h read W1
+// again, and the launch is bound by the latency of those reads from L2, not by arithmetic). Rounding points follow the two
+// conv_fused calls the reference issues on [N,C,1,1] tensors.
+static constexpr int SE_THREADS = 256;
+static constexpr int SE_ROW_LANES = 8;      // lanes per row of W1: 128 contiguous bytes per step
+__global__ void __launch_bounds__(SE_THREADS)
+se_gate_kernel(const void* __restrict__ g_in, const __half* __restrict__ w1, const __half* __restrict__ b1,
+               const __half* __restrict__ w2, const __half* __restrict__ b2, __half* __restrict__ s_out, int C, int Cs, int act,
+               float mean_scale, int slots, int cluster, int per, int sgroups) {
     extern __shared__ float sm[];
-    float* g = sm;          // [C]
-    float* h = sm + C;      // [Cs]
-    const long long n = blockIdx.x;
+    float* g = sm;                           // [per]
+    float* hp = g + per;                     // [cluster][Cs]: partial rows, one run per CTA of the cluster
+    float* h = hp + cluster * Cs;            // [Cs]
+    float* part = h + Cs;                    // [sgroups][per]
+    const int rank = static_cast<int>(cluster_ctarank());
+    const long long n = blockIdx.x / cluster;
+    const int c0 = rank * per, nc = max(0, min(per, C - c0));
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");      // this CTA runs: the others may write its `hp`
+    pdl_wait();
+    pdl_trigger();
     if (mean_scale != 0.f) {
         // fused squeeze: fp32 partial sums [slots][C] of this image times 1 / pixels. The slots are cut into `sgroups`
         // contiguous runs that are summed in parallel (every thread busy, several loads in flight), then the runs are
         // added in order: a fixed summation order, whatever the scheduling.
-        const float* gs = static_cast<const float*>(g_in) + n * slots * C;
-        float* part = sm + C + Cs;                 // [sgroups][C]
+        const float* gs = static_cast<const float*>(g_in) + n * slots * C + c0;
         const int run = (slots + sgroups - 1) / sgroups;
-        for (int idx = threadIdx.x; idx < C * sgroups; idx += blockDim.x) {
-            const int sg = idx / C, c = idx - sg * C;
+        for (int idx = threadIdx.x; idx < nc * sgroups; idx += SE_THREADS) {
+            const int sg = idx / nc, c = idx - sg * nc;
             const int k1 = min(slots, (sg + 1) * run);
             float sum = 0.f;
 #pragma unroll 8
-            for (int k = sg * run; k < k1; ++k) sum += gs[static_cast<long long>(k) * C + c];
-            part[idx] = sum;
+            for (int k = sg * run; k < k1; ++k) sum += __ldcg(gs + static_cast<long long>(k) * C + c);
+            part[sg * per + c] = sum;
         }
         __syncthreads();
-        for (int c = threadIdx.x; c < C; c += blockDim.x) {
+        for (int c = threadIdx.x; c < nc; c += SE_THREADS) {
             float sum = part[c];
-            for (int sg = 1; sg < sgroups; ++sg) sum += part[sg * C + c];
+            for (int sg = 1; sg < sgroups; ++sg) sum += part[sg * per + c];
             g[c] = __half2float(__float2half_rn(sum * mean_scale));
         }
     } else {
-        const __half* gh = static_cast<const __half*>(g_in) + n * C;
-        for (int c = threadIdx.x; c < C; c += blockDim.x) g[c] = __half2float(gh[c]);
+        const __half* gh = static_cast<const __half*>(g_in) + n * C + c0;
+        for (int c = threadIdx.x; c < nc; c += SE_THREADS)
+            g[c] = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(gh) + c)));
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int cv = C >> 3;
-    // FC1: a warp takes two rows of W1 at a time (eight 16-byte loads in flight per lane: the rows come from L2 and the
-    // loop is bound by that latency, not by arithmetic); each row's products are added in the same order as one by one
-    for (int j = 2 * warp; j < Cs; j += 2 * nwarps) {
-        const bool two = j + 1 < Cs;
-        const __half* row0 = w1 + static_cast<long long>(j) * C;
-        const __half* row1 = row0 + (two ? C : 0);
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int sub = lane / SE_ROW_LANES, sl = lane % SE_ROW_LANES;
+    const int nv = nc >> 3;
+    constexpr int ROWS = (SE_THREADS / 32) * (32 / SE_ROW_LANES);
+    for (int j0 = 0; j0 < Cs; j0 += 2 * ROWS) {          // two rows per lane group: their loads are in flight together
+        const int j = j0 + warp * (32 / SE_ROW_LANES) + sub, j2 = j + ROWS;
+        const __half* row0 = w1 + static_cast<long long>(min(j, Cs - 1)) * C + c0;
+        const __half* row1 = w1 + static_cast<long long>(min(j2, Cs - 1)) * C + c0;
         float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll 4
-        for (int v = lane; v < cv; v += 32) {
+        for (int v = sl; v < nv; v += SE_ROW_LANES) {
             float f0[8], f1[8];
             to_f8(ldg16(row0 + v * 8), f0);
             to_f8(ldg16(row1 + v * 8), f1);
@@ -276,25 +299,28 @@ __global__ void se_gate_kernel(const void* __restrict__ g_in, const __half* __re
             }
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int o = SE_ROW_LANES / 2; o > 0; o >>= 1) {
             acc0 += __shfl_xor_sync(0xffffffffu, acc0, o);
             acc1 += __shfl_xor_sync(0xffffffffu, acc1, o);
         }
-        if (lane == 0) {
-            if (b1) acc0 += __half2float(b1[j]);
-            h[j] = __half2float(__float2half_rn(act_f(acc0, act)));
-            if (two) {
-                if (b1) acc1 += __half2float(b1[j + 1]);
-                h[j + 1] = __half2float(__float2half_rn(act_f(acc1, act)));
-            }
+        if (sl < cluster) {                              // lane q of the group sends the sums to CTA q
+            const uint32_t dst = mapa_shared(smem_u32(hp + rank * Cs), static_cast<uint32_t>(sl));
+            if (j < Cs) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + 4u * j), "f"(acc0) : "memory");
+            if (j2 < Cs) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + 4u * j2), "f"(acc1) : "memory");
         }
+    }
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    for (int j = threadIdx.x; j < Cs; j += SE_THREADS) {
+        float acc = hp[j];
+        for (int q = 1; q < cluster; ++q) acc += hp[q * Cs + j];
+        if (b1) acc += __half2float(b1[j]);
+        h[j] = __half2float(__float2half_rn(act_f(acc, act)));
     }
     __syncthreads();
     // FC2: one output per thread and pass; the row of W2 (Cs halves) is fetched with all its loads in flight
     const int sv = Cs >> 3;
-    const int per = (C + gridDim.y - 1) / gridDim.y, c_end = min(C, static_cast<int>(blockIdx.y + 1) * per);
-    for (int c = blockIdx.y * per + threadIdx.x; c < c_end; c += blockDim.x) {
-        const __half* row = w2 + static_cast<long long>(c) * Cs;
+    for (int c = threadIdx.x; c < nc; c += SE_THREADS) {
+        const __half* row = w2 + static_cast<long long>(c0 + c) * Cs;
         float acc = 0.f;
         for (int v0 = 0; v0 < sv; v0 += 8) {
             uint4 q[8];
@@ -311,8 +337,8 @@ __global__ void se_gate_kernel(const void* __restrict__ g_in, const __half* __re
                 }
             }
         }
-        if (b2) acc += __half2float(b2[c]);
-        s_out[n * C + c] = __float2half_rn(acc);
+        if (b2) acc += __half2float(b2[c0 + c]);
+        s_out[n * C + c0 + c] = __float2half_rn(acc);
     }
 }
 
@@ -320,14 +346,16 @@ __global__ void se_gate_kernel(const void* __restrict__ g_in, const __half* __re
 // to fp16, fp16 multiply.
 __global__ void se_scale_kernel(const __half* __restrict__ x, const __half* __restrict__ s, __half* __restrict__ y,
                                 int HW, int C, long long total) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= total) return;
     const int cv = C >> 3;
     const int v = static_cast<int>(i % cv);
     const long long n = i / (static_cast<long long>(cv) * HW);
     V8 a, g, o;
-    a.u = ldg16(x + i * 8);
-    g.u = ldg16(s + n * C + v * 8);
+    a.u = ld16(x + i * 8);
+    g.u = ld16(s + n * C + v * 8);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float2 t = __half22float2(g.h2[j]);
@@ -344,6 +372,8 @@ __global__ void se_scale_kernel(const __half* __restrict__ x, const __half* __re
 // the other operand of the products instead, so that the scaled activation tensor is never written or re-read.
 __global__ void gate_weights_kernel(const __half* __restrict__ w, const __half* __restrict__ s, __half* __restrict__ out,
                                     int K, int C, long long total) {
+    pdl_wait();
+    pdl_trigger();
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;     // one 8-channel vector
     if (i >= total) return;
     const int cv = C >> 3;
@@ -353,7 +383,7 @@ __global__ void gate_weights_kernel(const __half* __restrict__ w, const __half* 
     const long long n = t / K;
     V8 a, g, o;
     a.u = ldg16(w + (static_cast<long long>(k) * C + v * 8));
-    g.u = ldg16(s + n * C + v * 8);
+    g.u = ld16(s + n * C + v * 8);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const float2 f = __half22float2(g.h2[j]);
@@ -373,6 +403,8 @@ template <int G, int VPL, int RPG>
 __global__ void __launch_bounds__(256)
 layernorm_cl_kernel(const __half* __restrict__ x, const __half* __restrict__ gamma, const __half* __restrict__ beta,
                     __half* __restrict__ y, long long rows, int C, float eps, long long ldx, long long ldy) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int GROUPS = 32 / G;
     const int warp_in_block = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane / G, gl = lane % G;
@@ -386,7 +418,7 @@ layernorm_cl_kernel(const __half* __restrict__ x, const __half* __restrict__ gam
         for (int k = 0; k < VPL; ++k) {
             const int v = gl + k * G;
             if (row0 + r < rows && v < cv) {
-                to_f8(ldg16(x + (row0 + r) * ldx + v * 8), f[r][k]);
+                to_f8(ld16(x + (row0 + r) * ldx + v * 8), f[r][k]);
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) f[r][k][j] = 0.f;
@@ -831,17 +863,13 @@ static int gap_launch(const void* x, void* y, float* partial, int N, int HW, int
     const int chunk = (HW + splits - 1) / splits;
     const float inv_hw = 1.f / static_cast<float>(HW);
     dim3 grid(((C >> 3) + GAP_VX - 1) / GAP_VX, splits, N), block(GAP_VX, GAP_RY);
-    gap_partial_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(x), partial, HW, C, ldx, splits, chunk, splits == 1 ? static_cast<__half*>(y) : nullptr,
-        inv_hw);
-    count_launch();
-    if (splits > 1) {
-        const long long total = static_cast<long long>(N) * C;
-        gap_final_kernel<<<blocks_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            partial, static_cast<__half*>(y), C, splits, inv_hw, total);
-        count_launch();
-    }
-    return cudaGetLastError() == cudaSuccess ? FVM_OK : FVM_ERR_LAUNCH;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int rc = launch_pdl(gap_partial_kernel, grid, block, 0, st, 1, static_cast<const __half*>(x), partial, HW, C, ldx, splits,
+                              chunk, splits == 1 ? static_cast<__half*>(y) : static_cast<__half*>(nullptr), inv_hw);
+    if (rc != FVM_OK || splits == 1) return rc;
+    const long long total = static_cast<long long>(N) * C;
+    return launch_pdl(gap_final_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, st, 1, static_cast<const float*>(partial),
+                      static_cast<__half*>(y), C, splits, inv_hw, total);
 }
 
 extern "C" int fvm_global_avgpool_f16(const void* x, void* y, float* partial, int N, int HW, int C, long long ldx,
@@ -859,24 +887,24 @@ static int se_gate_launch(const void* g, int slots, const void* w1, const void* 
     if (!g || !w1 || !w2 || !s || N <= 0 || C <= 0 || Cs <= 0 || (C & 7) || (Cs & 7) || act < 0 || act > 6 || slots < 1 ||
         !aligned16(w1) || !aligned16(w2))
         return FVM_ERR_ARG;
-    // runs of slots summed in parallel: enough to keep all threads busy, within the static shared-memory limit
-    int sgroups = mean_scale != 0.f ? slots / 16 : 0;
-    if (mean_scale != 0.f && sgroups < 1) sgroups = 1;
-    if (sgroups > 8) sgroups = 8;
-    while (sgroups > 1 && static_cast<size_t>(C) * (1 + sgroups) + Cs > 12 * 1024 - 64) --sgroups;
-    const size_t smem = (static_cast<size_t>(C) * (1 + sgroups) + Cs) * sizeof(float);
-    if (smem > 48 * 1024) return FVM_ERR_ARG;
+    if (static_cast<size_t>(C) * (mean_scale != 0.f ? 2 : 1) + Cs > 12 * 1024) return FVM_ERR_ARG;
     DeviceState* st = device_state();
     const int sms = st ? st->sms : 148;
-    // large layers: 1024 threads (the loops are latency-bound: more rows / outputs in flight per SM), one block per SM
-    const int threads = static_cast<long long>(C) * Cs >= 16 * 1024 ? 1024 : 256;
-    const int resident = threads == 1024 ? sms : 2 * sms;
-    int split = 1;                       // blocks per image: fill the GPU when the batch alone does not, in one wave
-    while (split < 4 && N * split * 2 <= resident && C / (split * 2) >= 256) split *= 2;
-    se_gate_kernel<<<dim3(N, split), threads, smem, static_cast<cudaStream_t>(stream)>>>(
-        g, static_cast<const __half*>(w1), static_cast<const __half*>(b1), static_cast<const __half*>(w2),
-        static_cast<const __half*>(b2), static_cast<__half*>(s), C, Cs, act, mean_scale, slots, sgroups);
-    FVM_LAUNCH_CHECK();
+    // CTAs per image: as many as stay resident at once (four blocks of 256 threads per SM) with 64 channels or more each
+    int cluster = 8;
+    while (cluster > 1 && (static_cast<long long>(N) * cluster > 4ll * sms || C < 64 * cluster)) cluster >>= 1;
+    const int per = ((C >> 3) + cluster - 1) / cluster * 8;
+    int sgroups = mean_scale != 0.f ? SE_THREADS / per : 0;       // runs of slots summed in parallel: every thread busy
+    if (mean_scale != 0.f && sgroups < 1) sgroups = 1;
+    if (sgroups > slots) sgroups = slots;
+    const size_t smem = (static_cast<size_t>(per) * (1 + sgroups) + static_cast<size_t>(cluster + 1) * Cs) * sizeof(float);
+    if (smem > 200 * 1024) return FVM_ERR_ARG;
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(se_gate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
+        return FVM_ERR_SETUP;
+    if (static_cast<long long>(N) * cluster > 0x7fffffffll) return FVM_ERR_ARG;
+    return launch_pdl(se_gate_kernel, dim3(static_cast<unsigned>(N * cluster)), dim3(SE_THREADS), smem, static_cast<cudaStream_t>(stream),
+                      cluster, g, static_cast<const __half*>(w1), static_cast<const __half*>(b1), static_cast<const __half*>(w2),
+                      static_cast<const __half*>(b2), static_cast<__half*>(s), C, Cs, act, mean_scale, slots, cluster, per, sgroups);
 }
 
 extern "C" int fvm_se_gate_f16(const void* g, const void* w1, const void* b1, const void* w2, const void* b2, void* s,
@@ -895,42 +923,39 @@ extern "C" int fvm_gate_weights_f16(const void* w, const void* s, void* out, int
     if (!w || !s || !out || N <= 0 || K <= 0 || C <= 0 || (C & 7) || !aligned16(w) || !aligned16(s) || !aligned16(out))
         return FVM_ERR_ARG;
     const long long total = static_cast<long long>(N) * K * (C >> 3);
-    gate_weights_kernel<<<blocks_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(w), static_cast<const __half*>(s), static_cast<__half*>(out), K, C, total);
-    FVM_LAUNCH_CHECK();
+    return launch_pdl(gate_weights_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, static_cast<cudaStream_t>(stream), 1,
+                      static_cast<const __half*>(w), static_cast<const __half*>(s), static_cast<__half*>(out), K, C, total);
 }
 
 extern "C" int fvm_se_scale_f16(const void* x, const void* s, void* y, int N, int HW, int C, void* stream) {
     if (!x || !s || !y || N <= 0 || HW <= 0 || C <= 0 || (C & 7) || !aligned16(x) || !aligned16(y) || !aligned16(s))
         return FVM_ERR_ARG;
     const long long total = static_cast<long long>(N) * HW * (C >> 3);
-    se_scale_kernel<<<blocks_for(total, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __half*>(x), static_cast<const __half*>(s), static_cast<__half*>(y), HW, C, total);
-    FVM_LAUNCH_CHECK();
+    return launch_pdl(se_scale_kernel, dim3(blocks_for(total, 256)), dim3(256), 0, static_cast<cudaStream_t>(stream), 1,
+                      static_cast<const __half*>(x), static_cast<const __half*>(s), static_cast<__half*>(y), HW, C, total);
 }
 
 template <int G, int VPL>
-static void launch_ln(const void* x, const void* gamma, const void* beta, void* y, long long rows, int C, float eps,
+static int launch_ln(const void* x, const void* gamma, const void* beta, void* y, long long rows, int C, float eps,
                       long long ldx, long long ldy, cudaStream_t stream) {
     constexpr int RPG = VPL >= 3 ? 2 : 4;           // rows in flight per lane group (registers: RPG * VPL * 8 floats)
     constexpr int WARPS = 4;
     const long long rows_per_block = static_cast<long long>(WARPS) * (32 / G) * RPG;
-    layernorm_cl_kernel<G, VPL, RPG><<<blocks_for(rows, static_cast<int>(rows_per_block)), WARPS * 32, 0, stream>>>(
-        static_cast<const __half*>(x), static_cast<const __half*>(gamma), static_cast<const __half*>(beta),
-        static_cast<__half*>(y), rows, C, eps, ldx, ldy);
-    count_launch();
+    return launch_pdl(layernorm_cl_kernel<G, VPL, RPG>, dim3(blocks_for(rows, static_cast<int>(rows_per_block))), dim3(WARPS * 32), 0,
+                      stream, 1, static_cast<const __half*>(x), static_cast<const __half*>(gamma), static_cast<const __half*>(beta),
+                      static_cast<__half*>(y), rows, C, eps, ldx, ldy);
 }
 
 template <int G>
-static bool launch_ln_g(int vpl, const void* x, const void* gamma, const void* beta, void* y, long long rows, int C,
+static int launch_ln_g(int vpl, const void* x, const void* gamma, const void* beta, void* y, long long rows, int C,
                         float eps, long long ldx, long long ldy, cudaStream_t st) {
     switch (vpl) {
-        case 1: launch_ln<G, 1>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st); return true;
-        case 2: launch_ln<G, 2>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st); return true;
-        case 3: launch_ln<G, 3>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st); return true;
-        case 4: launch_ln<G, 4>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st); return true;
+        case 1: return launch_ln<G, 1>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+        case 2: return launch_ln<G, 2>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+        case 3: return launch_ln<G, 3>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+        case 4: return launch_ln<G, 4>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
     }
-    return false;
+    return FVM_ERR_ARG;
 }
 
 extern "C" int fvm_layernorm_cl_f16(const void* x, const void* gamma, const void* beta, void* y, long long rows, int C,
@@ -941,15 +966,13 @@ extern "C" int fvm_layernorm_cl_f16(const void* x, const void* gamma, const void
     const int cv = C >> 3;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // smallest lane group whose lanes hold at most 4 vectors each; rows wider than 128 vectors: 32 lanes x 6 or 8
-    bool ok = false;
-    if (cv <= 16) ok = launch_ln_g<4>((cv + 3) / 4, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
-    else if (cv <= 32) ok = launch_ln_g<8>((cv + 7) / 8, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
-    else if (cv <= 64) ok = launch_ln_g<16>((cv + 15) / 16, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
-    else if (cv <= 128) ok = launch_ln_g<32>((cv + 31) / 32, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
-    else if (cv <= 192) { launch_ln<32, 6>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st); ok = true; }
-    else if (cv <= 256) { launch_ln<32, 8>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st); ok = true; }
-    if (!ok) return FVM_ERR_ARG;
-    return cudaGetLastError() == cudaSuccess ? FVM_OK : FVM_ERR_LAUNCH;
+    if (cv <= 16) return launch_ln_g<4>((cv + 3) / 4, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+    if (cv <= 32) return launch_ln_g<8>((cv + 7) / 8, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+    if (cv <= 64) return launch_ln_g<16>((cv + 15) / 16, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+    if (cv <= 128) return launch_ln_g<32>((cv + 31) / 32, x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+    if (cv <= 192) return launch_ln<32, 6>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+    if (cv <= 256) return launch_ln<32, 8>(x, gamma, beta, y, rows, C, eps, ldx, ldy, st);
+    return FVM_ERR_ARG;
 }
 
 extern "C" int fvm_bias_act_f16(void* y, const void* bias, const void* res, long long pixels, int C, int relu,

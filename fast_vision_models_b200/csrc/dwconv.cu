@@ -69,11 +69,14 @@ __device__ __forceinline__ void dw_stage_issue(const CUtensorMap* tmap, const Dw
         *abort_flag = 0;
         mbar_init(bar, 1);
         mbar_fence_init();
+        pdl_wait();       // the copy below is the block's first access to the input
         mbar_expect_tx(bar, static_cast<uint32_t>(p.tile_h * p.tile_w * p.cbv) * 16u);
         tma_load_4d(smem0, tmap, bar, vb * p.cbv * 8, w0, h0, n);
     }
 }
 __device__ __forceinline__ bool dw_stage_wait(const DwParams& p, uint32_t bar, volatile int* abort_flag) {
+    pdl_wait();           // every thread: the outputs may still be read by an earlier kernel
+    pdl_trigger();
     __syncthreads();
     if (!mbar_wait<32>(bar, 0u, abort_flag)) {
         if (threadIdx.x == 0) atomicExch(p.status, STATUS_WAIT_DW);
@@ -424,7 +427,7 @@ extern "C" int fvm_dwconv_f16(const void* x, const void* w_rsc, const void* bias
         if (plan.smem > 48 * 1024 &&                                                                                  \
             cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, DW_SMEM_LIMIT) != cudaSuccess)  \
             return FVM_ERR_SETUP;                                                                                     \
-        KERNEL<<<grid, DW_THREADS, plan.smem, s>>>(tmap, wp, bp, yp, pool_partial, p);                                \
+        return launch_pdl(KERNEL, grid, dim3(DW_THREADS), plan.smem, s, 1, tmap, wp, bp, yp, pool_partial, p);        \
     } while (0)
 #define DW_ACT_TW(SV, SWV, TWV)                                               \
     do {                                                                      \
@@ -444,6 +447,4 @@ extern "C" int fvm_dwconv_f16(const void* x, const void* w_rsc, const void* bias
 #undef DW_ACT
 #undef DW_ACT_TW
 #undef DW_LAUNCH
-    count_launch();
-    return cudaGetLastError() == cudaSuccess ? FVM_OK : FVM_ERR_LAUNCH;
 }

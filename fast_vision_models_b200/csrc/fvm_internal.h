@@ -72,4 +72,30 @@ int conv_dual_launch(const void* x, const void* w1, const void* b1, const void* 
                      void* z, long long M, int C1, int K1, int K2, long long ldx, long long ldr, long long ldy, long long ldz,
                      int act1, int act2, cudaStream_t stream);
 
+// Launch with programmatic stream serialization (the kernel calls pdl_wait before it touches activations) in clusters of
+// `cluster` blocks. Measured on B200 in a replayed graph: a plain launch adds about 1 us between two small kernels.
+template <typename... P, typename... A>
+int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = 1;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attrs[1].val.clusterDim.y = 1;
+    attrs[1].val.clusterDim.z = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return FVM_ERR_LAUNCH;
+    }
+    count_launch();
+    return FVM_OK;
+}
+
 }  // namespace fvm

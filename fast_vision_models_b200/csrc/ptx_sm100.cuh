@@ -20,6 +20,13 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// Before the first access to anything an earlier kernel of the stream wrote or still reads; no-op in a plain launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel may start its set-up. After pdl_wait in kernels that read activations through L1: a kernel started from
+// here on then starts (with a clean L1) after everything before this kernel has finished.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

@@ -916,6 +916,25 @@ def test_se_gate_and_scale_match_oracle(N, C, Cs, act):
     close(ops.se_scale(cl(x), ref_s.to(DEV)), R.se_scale_ref(x, ref_s))
 
 
+@pytest.mark.parametrize("case", [
+    # N, C, Cs, slots, act: clusters of 8, 4, 2 and 1 CTAs per image
+    (1, 1152, 48, 4, 3), (2, 520, 24, 1, 1), (150, 264, 8, 3, 3), (300, 136, 16, 2, 3), (601, 72, 8, 5, 3), (1, 8, 8, 70, 0),
+    (3, 5120, 40, 2, 3),
+])
+def test_se_gate_clusters_match_oracle(case):
+    N, C, Cs, slots, act = case
+    g = torch.Generator().manual_seed(91)
+    partial = torch.rand((N, slots, C), generator=g) * 4 - 1
+    w1, b1 = gen((Cs, C), 92, C ** -0.5), gen((Cs,), 93, 0.1)
+    w2, b2 = gen((C, Cs), 94, Cs ** -0.5), gen((C,), 95, 0.1)
+    mean = (partial.sum(1) / (slots * 4.0)).half().view(N, C, 1, 1)
+    ref = R.se_gate_ref(mean, w1, b1, w2, b2, act)
+    s = ops.se_gate_pooled(partial.to(DEV), slots * 4, w1.to(DEV), b1.to(DEV), w2.to(DEV), b2.to(DEV), act)
+    close(s, ref, 2e-3)                       # two fp16 roundings on the way, as the plain gate's test
+    assert torch.equal(s, ops.se_gate_pooled(partial.to(DEV), slots * 4, w1.to(DEV), b1.to(DEV), w2.to(DEV), b2.to(DEV), act))
+    close(ops.se_gate(mean.to(DEV), w1.to(DEV), b1.to(DEV), w2.to(DEV), b2.to(DEV), act), ref, 2e-3)
+
+
 @pytest.mark.parametrize("case", [(3, 144, 19, 19, 24, False), (4, 672, 24, 24, 112, True), (2, 48, 7, 5, 40, True),
                                   (64, 960, 12, 12, 272, False), (5, 96, 1, 1, 32, False)])
 def test_gate_folded_into_project_weights_matches_scale_then_conv(case):
