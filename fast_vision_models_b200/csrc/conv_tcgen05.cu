@@ -2719,17 +2719,20 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
     if (!x || !w || !y) return FVM_ERR_ARG;
     // force_bn: low 16 bits = output-channel tile (0 = choose), bits 16..23 = sub-tiles per tile (0 = choose),
     // bits 24..25 = weight-resident mode (0 = choose, 1 = on, 2 = off), bits 26..27 = halo mode, bits 28..29 = stream-K
-    // (same coding; 3 = conv_split_kernel with the CTAs per tile in bits 16..23), bit 30 = CTA pairs (conv_pair_kernel) on
+    // (same coding; 3 = conv_split_kernel with the CTAs per tile in bits 16..23, with bit 30 CTA pairs per tile), bit 30 = CTA
+    // pairs (conv_pair_kernel) on
     int force_pair = force_bn > 0 ? ((force_bn >> 30) & 1) : 0;
     const bool free_choice = force_bn <= 0;
     int force_sk = force_bn > 0 ? ((force_bn >> 28) & 3) : 0;
     int force_halo = force_bn > 0 ? ((force_bn >> 26) & 3) : 0;
     const int force_bres = force_bn > 0 ? ((force_bn >> 24) & 3) : 0;
     int force_mt = force_bn > 0 ? ((force_bn >> 16) & 0xff) : 0;
-    int split = 0, wdyn = 0;        // conv_split_kernel: CTAs per tile (0: not used); weights not constant
+    int split = 0, split_pair = 0, wdyn = 0;        // conv_split_kernel: CTAs (CTA pairs) per tile (0: not used); weights not constant
     if (force_sk == 3) {
         split = force_mt;
-        if (split <= 0 || force_pair || force_halo == 1 || force_bres == 1 || gsg > 0) return FVM_ERR_ARG;
+        split_pair = force_pair;
+        force_pair = 0;
+        if (split <= 0 || (split_pair && st->pair_clusters <= 0) || force_halo == 1 || force_bres == 1 || gsg > 0) return FVM_ERR_ARG;
         force_sk = force_mt = 0;
     }
     force_bn = force_bn > 0 ? (force_bn & 0xffff) : 0;
@@ -2930,7 +2933,7 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
             p.bres = 1;
     }
     if (force_bres == 1 && !p.bres) return FVM_ERR_ARG;
-    if (!plan_smem(p.BN, p.mt, p.kblocks, K, p.tapk != 0, p.bres != 0, &sp, halo_bytes, p.pair != 0)) return FVM_ERR_ARG;
+    if (!plan_smem(p.BN, p.mt, p.kblocks, K, p.tapk != 0, p.bres != 0, &sp, halo_bytes, p.pair || split_pair)) return FVM_ERR_ARG;
     p.bias_elems = p.n_tiles * p.BN;
     p.stages = sp.stages;
     p.nepi = sp.nepi;
@@ -3023,7 +3026,7 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
         cuuint64_t dims[3] = {static_cast<cuuint64_t>(Cw), static_cast<cuuint64_t>(R * S),
                               static_cast<cuuint64_t>(K) * (p.wb ? N : 1)};
         cuuint64_t strides[2] = {static_cast<cuuint64_t>(Cw) * 2, static_cast<cuuint64_t>(R) * S * Cw * 2};
-        cuuint32_t box[3] = {static_cast<cuuint32_t>(p.tapk ? p.tapk : BK), 1, static_cast<cuuint32_t>(p.pair ? p.BN / 2 : p.BN)};
+        cuuint32_t box[3] = {static_cast<cuuint32_t>(p.tapk ? p.tapk : BK), 1, static_cast<cuuint32_t>(p.pair || split_pair ? p.BN / 2 : p.BN)};
         cuuint32_t estr[3] = {1, 1, 1};
         CUresult r = g_encode_tiled(&tmap_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(w), dims, strides,
                                     box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -3093,7 +3096,7 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
         q.M = p.M; q.K = K; q.P = P; q.Q = Q; q.S = S;
         q.sh = sh; q.sw = sw; q.ph = ph; q.pw = pw; q.dh = dh; q.dw = dw;
         q.cchunks = p.cchunks; q.kblocks = p.kblocks; q.im2col = p.im2col;
-        q.BN = p.BN; q.n_tiles = p.n_tiles; q.split = split;
+        q.BN = p.BN; q.n_tiles = p.n_tiles; q.split = split; q.pair = split_pair;
         q.act = act;
         q.wdyn = wdyn;
         q.bias = p.bias;

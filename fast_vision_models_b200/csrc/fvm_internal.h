@@ -42,11 +42,12 @@ int conv2d_launch(const void* x, const void* w, const void* bias, const void* re
                   int H, int W, int C, int K, int R, int S, int ph, int pw, int sh, int sw, int dh, int dw,
                   long long ldx, long long ldy, long long ldr, int act, int force_bn, int ph_hi, int pw_hi,
                   cudaStream_t stream, int w_per_image = 0, int gsg = 0, int gsk = 0);
-// Cluster split-K convolution (conv_split.cu): one 128 x BN output tile per cluster of `split` CTAs.
+// Cluster split-K convolution (conv_split.cu): one output tile per cluster of `split` CTAs or CTA pairs.
 struct SplitParams {
     int M, K, P, Q, S, sh, sw, ph, pw, dh, dw;
     int cchunks, kblocks, im2col;
     int BN, n_tiles, split;
+    int pair;                          // tiles of 256 x BN, `split` CTA pairs per cluster (conv_split_pair_kernel)
     int lg_bn, stages, tmem_cols;      // from conv_split_plan
     uint32_t red_bytes;
     int act;

@@ -210,6 +210,9 @@ class FusedConv(nn.Module):
             for c in (64, 128):
                 tiles = ((rows + 127) // 128) * ((K + c - 1) // c)
                 cands += [(3 << 28) | (n << 16) | c for n in (2, 3, 4, 6, 8) if n <= kblocks and tiles * n <= 148]
+            for c in (128, 256):          # deep reductions: clusters of CTA pairs (bit 30), tiles of 256 pixels
+                tiles = ((rows + 255) // 256) * ((K + c - 1) // c)
+                cands += [(1 << 30) | (3 << 28) | (n << 16) | c for n in (2, 3, 4) if 32 * n <= kblocks and tiles * 2 * n <= 148]
         best = 0
         if len(cands) > 1:
             # Candidates are timed in rounds (every candidate once per round, best burst kept), so that a drift of the

@@ -82,7 +82,8 @@ int fvm_conv2d_f16(const void* x, const void* w, const void* bias, const void* r
  * bit for bit; not with sub-tiles, halo, weight-resident or stream-K mode). Bits 28..29 = 3: each tile of 128 pixels x tile_n
  * channels (32, 64 or 128) is shared by a cluster of as many CTAs as bits 16..23 say (1 to 8, at most one per 64-channel
  * k-block; tile_n at most 64 times as wide as there are CTAs), which split the reduction and add their fp32 partial sums in a
- * fixed order (for layers with few tiles; not with the other modes). Shapes that do not fit return 1. */
+ * fixed order (for layers with few tiles; not with the other modes); with bit 30 as well, tiles of 256 pixels x 64, 128 or 256
+ * channels and clusters of 2 to 4 CTA pairs. Shapes that do not fit return 1. */
 int fvm_conv2d_f16_tile(const void* x, const void* w, const void* bias, const void* res, const float* scale, void* y,
                         int N, int H, int W, int C, int K, int R, int S, int ph, int pw, int sh, int sw, int dh, int dw,
                         long long ldx, long long ldy, long long ldr, int act, int tile_n, void* stream);

@@ -283,7 +283,7 @@ def test_conv_cta_pairs_are_refused_where_they_do_not_apply():
 
 
 @pytest.mark.parametrize("case", [
-    # N, H, W, C, K, R, pad, stride, dil, res, scale, act, bn, split
+    # N, H, W, C, K, R, pad, stride, dil, res, scale, act, bn, split (negative: CTA pairs)
     (1, 7, 7, 512, 512, 3, 1, 1, 1, False, False, 1, 64, 8),        # 49 of 128 rows, slices of 7 rows (the last has none to do)
     (1, 14, 14, 256, 256, 3, 1, 2, 1, True, False, 1, 64, 7),       # uneven runs of k-blocks, residual
     (3, 13, 17, 72, 136, 3, 2, 1, 2, True, True, 5, 128, 6),        # dilation, ragged channels, tiles over images, fp32 scale
@@ -291,6 +291,10 @@ def test_conv_cta_pairs_are_refused_where_they_do_not_apply():
     (2, 1, 1, 2048, 1000, 1, 0, 1, 1, False, False, 2, 128, 5),     # two rows for five CTAs
     (1, 12, 11, 24, 24, 1, 0, 1, 1, True, False, 3, 32, 1),         # a single k-block, 24 of 32 columns, a second tile of 4 rows
     (2, 16, 16, 320, 200, 1, 0, 1, 1, True, False, 6, 128, 2),      # 64 rows per CTA: the most units per thread
+    (1, 7, 7, 512, 512, 3, 1, 1, 1, False, False, 1, 256, -4),      # pairs: the odd CTA has no row at all
+    (2, 14, 14, 256, 264, 3, 1, 1, 1, True, False, 1, 256, -2),     # two chunks of units per thread, a tile 8 columns wide, odd CTA partly empty
+    (3, 13, 17, 72, 136, 3, 2, 1, 2, True, True, 5, 64, -3),        # uneven runs and slices, dilation, tiles over images, fp32 scale
+    (5, 16, 16, 2048, 512, 1, 0, 1, 1, False, False, 3, 128, -4),   # five full tiles of 256 pixels, SiLU
 ])
 def test_conv_split_matches_oracle(case):
     # one tile per cluster, the reduction split over its CTAs: against the oracle, and the same bits twice in a row (the
@@ -302,7 +306,7 @@ def test_conv_split_matches_oracle(case):
     r = gen((N, K, P, Q), 74) if res else None
     sc = torch.rand(K, generator=torch.Generator().manual_seed(75)) + 0.5 if scale else None
     ref = R.conv_fused_ref(x, w, b, r, (pad, pad), (stride, stride), act, (dil, dil), sc)
-    code = (3 << 28) | (split << 16) | bn
+    code = (3 << 28) | (abs(split) << 16) | bn | ((1 << 30) if split < 0 else 0)
     args = (cl(x), cl(w), b.to(DEV), None if r is None else cl(r), (pad, pad), (stride, stride), act)
     kw = dict(dilation=(dil, dil), scale=None if sc is None else sc.to(DEV), tile_n=code)
     y = ops.conv_fused(*args, **kw)
