@@ -37,6 +37,10 @@ static constexpr int DW_THREADS = 128;
 // 119 us with 4 columns against 131 with 8; 5x5 C=336 48x48: 82 against 137 the other way round; 7x7 C=96 56x56: 64
 // against 76): narrow strips keep more CTAs on an SM, wide ones re-use each staged input vector for more outputs.
 static constexpr int dw_tw(int S) { return S == 5 ? 8 : 4; }
+// Layers whose blocks would not fill the GPU once (one image, above all) take strips of two columns: what they cost is the
+// serial work of a thread (one image, us: 56x56x144 5x5 stride 2 8.7 -> 4.6, 28x28x240 5x5 6.4 -> 3.7, 14x14x672 5x5 4.9 -> 3.7;
+// four images of the last, with 192 blocks already, 4.9 -> 5.0).
+static constexpr int DW_NARROW = 2;
 static constexpr int DW_SMEM_LIMIT = 96 * 1024; // per CTA: at least two CTAs per SM
 static constexpr int STATUS_WAIT_DW = 0x105;
 
@@ -195,22 +199,34 @@ dw_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __half* __restr
                 __align__(16) __half2 o[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    // the sum is rounded to fp16 first; relu acts on the fp16 pair, other activations are evaluated
-                    // in fp32 on the rounded value and rounded again (reference: r3.cu:404-413)
-                    o[k] = __floats2half2_rn(acc[j][2 * k], acc[j][2 * k + 1]);
-                    if (ACT == 1) {
-                        o[k] = __hmax2(o[k], __float2half2_rn(0.f));
-                    } else if (ACT == 3) {      // SiLU on the pair in fp32: packed multiplies, ex2 / rcp per element
-                        const uint32_t sv = f2_to_h2(f2_silu(h2_to_f2(*reinterpret_cast<const uint32_t*>(&o[k]))));
+                    // the sum is rounded to fp16 first; relu acts on the fp16 pair, other activations are evaluated in fp32
+                    // on the rounded value and rounded again (reference: r3.cu:404-413). SiLU with stride 1 takes the fp32
+                    // sums as they are: three instructions per pair and one rounding error less (batch 64, with the squeeze
+                    // sums by mixed-precision adds: 48x48x336 5x5 84.2 -> 80.7 us, 95x95x192 3x3 124.9 -> 122.3; with
+                    // stride 2 it was slower, 190x190x144 3x3 215 -> 224)
+                    if (ACT == 3 && SW == 1) {
+                        const uint32_t sv = f2_to_h2(f2_silu(f2_pack(__float_as_uint(acc[j][2 * k]), __float_as_uint(acc[j][2 * k + 1]))));
                         o[k] = *reinterpret_cast<const __half2*>(&sv);
-                    } else if (ACT != 0) {
-                        const float2 f = __half22float2(o[k]);
-                        o[k] = __floats2half2_rn(act_f(f.x, p.act), act_f(f.y, p.act));
+                    } else {
+                        o[k] = __floats2half2_rn(acc[j][2 * k], acc[j][2 * k + 1]);
+                        if (ACT == 1) {
+                            o[k] = __hmax2(o[k], __float2half2_rn(0.f));
+                        } else if (ACT == 3) {
+                            const uint32_t sv = f2_to_h2(f2_silu(h2_to_f2(*reinterpret_cast<const uint32_t*>(&o[k]))));
+                            o[k] = *reinterpret_cast<const __half2*>(&sv);
+                        } else if (ACT != 0) {
+                            const float2 f = __half22float2(o[k]);
+                            o[k] = __floats2half2_rn(act_f(f.x, p.act), act_f(f.y, p.act));
+                        }
                     }
                     if (pool_partial) {
-                        const float2 f = __half22float2(o[k]);
-                        psum[2 * k] += f.x;
-                        psum[2 * k + 1] += f.y;
+                        if (SW == 1) {
+                            f32_add_h2(psum[2 * k], psum[2 * k + 1], *reinterpret_cast<const uint32_t*>(&o[k]));
+                        } else {
+                            const float2 f = __half22float2(o[k]);
+                            psum[2 * k] += f.x;
+                            psum[2 * k + 1] += f.y;
+                        }
                     }
                 }
                 *reinterpret_cast<uint4*>(y + ((n * p.P + pr) * p.Q + q) * p.ldy + v * 8) = *reinterpret_cast<uint4*>(o);
@@ -304,13 +320,13 @@ static int pick_cbv(int cv) {
 
 struct DwPlan {
     DwParams p;
-    bool tile_kernel;
+    bool tile_kernel, narrow;
     size_t smem;
 };
 
 // Tile geometry for one layer: which kernel, the channel block, the cell grid and the staged patch.
 static bool dw_plan(int N, int H, int W, int C, int R, int S, int ph, int pw, int sh, int sw, int dh, int dw, long long ldy,
-                    int act, DwPlan* out) {
+                    int act, DwPlan* out, bool narrow = false) {
     DwParams& p = out->p;
     memset(&p, 0, sizeof(p));
     p.H = H; p.W = W; p.C = C; p.R = R; p.S = S;
@@ -327,7 +343,8 @@ static bool dw_plan(int N, int H, int W, int C, int R, int S, int ph, int pw, in
     // the one with the least staged bytes per output pixel (least border) is taken. Measured on B200: small CTAs win
     // over taller tiles with several output rows per thread (more CTAs per SM overlap one CTA's copy with the others'
     // arithmetic), so a thread keeps to one output row.
-    const int unit = out->tile_kernel ? dw_tw(S) : 1;
+    out->narrow = narrow && out->tile_kernel && S != 7;
+    const int unit = !out->tile_kernel ? 1 : out->narrow ? DW_NARROW : dw_tw(S);
     struct Cand { int cbv, px, py, tile_w, tile_h, tiles_x, tiles_y, vblocks; double score, cost; size_t bytes; };
     Cand cands[40];
     int nc = 0;
@@ -359,7 +376,12 @@ static bool dw_plan(int N, int H, int W, int C, int R, int S, int ph, int pw, in
     p.cbv = c.cbv; p.px = c.px; p.py = c.py; p.tile_w = c.tile_w; p.tile_h = c.tile_h;
     p.tiles_x = c.tiles_x; p.tiles_y = c.tiles_y; p.vblocks = c.vblocks;
     out->smem = 128 + c.bytes + 16 + static_cast<size_t>(DW_THREADS) * 8 * sizeof(float) + 6272;    // + up to 49 taps x 8 vectors of weights
-    (void)N;
+    const DeviceState* st = device_state();
+    if (out->tile_kernel && !narrow && S != 7 &&
+        static_cast<long long>(N) * p.tiles_x * p.tiles_y * p.vblocks < (st ? st->sms : 148)) {
+        DwPlan small;
+        if (dw_plan(N, H, W, C, R, S, ph, pw, sh, sw, dh, dw, ldy, act, &small, true)) *out = small;
+    }
     return true;
 }
 
@@ -436,11 +458,15 @@ extern "C" int fvm_dwconv_f16(const void* x, const void* w_rsc, const void* bias
         else if (act == 3) DW_LAUNCH((dw_tile_kernel<SV, SWV, 3, TWV>));      \
         else DW_LAUNCH((dw_tile_kernel<SV, SWV, -1, TWV>));                   \
     } while (0)
-#define DW_ACT(SV, SWV) DW_ACT_TW(SV, SWV, dw_tw(SV))
+#define DW_ACT(SV, SWV)                                           \
+    do {                                                          \
+        if (plan.narrow) DW_ACT_TW(SV, SWV, DW_NARROW);           \
+        else DW_ACT_TW(SV, SWV, dw_tw(SV));                       \
+    } while (0)
     if (plan.tile_kernel) {
         if (S == 3) { if (sw == 1) DW_ACT(3, 1); else DW_ACT(3, 2); }
         else if (S == 5) { if (sw == 1) DW_ACT(5, 1); else DW_ACT(5, 2); }
-        else DW_ACT(7, 2);
+        else DW_ACT_TW(7, 2, dw_tw(7));
     } else {
         DW_LAUNCH(dw_any_kernel);
     }

@@ -853,6 +853,17 @@ def test_dwconv_7x7_on_tensor_cores(case):
     assert (partial.sum(1).cpu() - sums).abs().max() <= 1e-5 * y.float().abs().sum((2, 3)).max().cpu() + 1e-5
 
 
+@pytest.mark.parametrize("case", [(k, stride, n) for k in (3, 5) for stride in (1, 2) for n in (1, 40)])
+def test_dwconv_strip_widths(case):
+    # few blocks: strips of two columns per thread, many: four or eight; 31 x 29 ends inside a strip either way
+    k, stride, n = case
+    x, w, b = gen((n, 72, 31, 29), 86), gen((k, k, 72), 87, 0.2), gen((72,), 88, 0.1)
+    ref = R.dwconv_ref(x, w, b, (stride, stride), (k // 2, k // 2), 3)
+    y = ops.dwconv(cl(x), w.to(DEV), b.to(DEV), (stride, stride), (k // 2, k // 2), 3)
+    assert ops.last_status() == 0
+    close(y, ref)
+
+
 @pytest.mark.parametrize("bad", [float("inf"), float("nan"), -float("inf")])
 def test_dwconv_7x7_non_finite_values_stay_in_their_windows(bad):
     # the zeros of the Toeplitz matrices must not meet an infinity or a NaN: exactly the outputs whose window holds it change
