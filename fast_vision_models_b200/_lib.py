@@ -129,6 +129,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
 def load() -> ctypes.CDLL:
     """Load the library, building it first when the sources changed. Raises if no current library can be had."""
     global _lib
+    if _lib is not None:          # set once, complete
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib

@@ -41,6 +41,8 @@ def lib() -> ctypes.CDLL:
 
 def init(device: Optional[torch.device] = None) -> None:
     """Per-device set-up; must run before the first launch on a device and before any CUDA-graph capture."""
+    if device is not None and device.index in _initialised_devices and torch._C._cuda_getDevice() == device.index:
+        return
     if not torch.cuda.is_available():
         raise FvmError("fvm_b200 needs a CUDA device (sm_100a); there is no CPU path")
     cur = torch.cuda.current_device()
@@ -95,7 +97,7 @@ def _stream() -> int:
     # anything else that could read their outputs
     if _chain is not None and _chain.layers:
         _chain.flush()
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 # ------------------------------------------------------------------------------------------------ layer chains
@@ -178,9 +180,10 @@ def nhwc_view(x: torch.Tensor, name: str = "x"):
     """Returns (tensor, N, C, H, W, ld): `tensor` is NHWC in memory with pixel stride `ld` (a channels-last tensor or a
     channel slice of one); anything else is made channels-last contiguous first (reference: fused_conv.cu:237-244)."""
     _require_cuda_half(x, name)
-    if x.dim() != 4:
+    shape = x.shape
+    if len(shape) != 4:
         raise FvmError(f"{name}: expected a 4-D NCHW-shaped tensor")
-    N, C, H, W = x.shape
+    N, C, H, W = shape
     sN, sC, sH, sW = x.stride()
     # pixel (n,h,w) must sit at ((n*H + h)*W + w) * ld; ld comes from the innermost dimension that has extent > 1
     if W > 1:
@@ -206,6 +209,8 @@ def empty_nhwc(N: int, C: int, H: int, W: int, device) -> torch.Tensor:
 
 
 def _pair(v) -> tuple:
+    if type(v) is tuple and len(v) == 2 and type(v[0]) is int and type(v[1]) is int:
+        return v
     if isinstance(v, int):
         return (v, v)
     v = tuple(int(a) for a in v)
@@ -226,6 +231,12 @@ def conv_fused_into(x, w, bias, res, padding, stride, act: int, out: torch.Tenso
     """clf::conv_fused_into / segx::conv_fused_into: y = act((conv(x,w)+bias)*scale + res) written into `out`.
     `pad_hi` = (bottom, right) padding when it differs from `padding` = (top, left)."""
     init(x.device)
+    _conv(x, w, bias, res, padding, stride, act, out, dilation, scale, tile_n, pad_hi)
+
+
+def _conv(x, w, bias, res, padding, stride, act, out: Optional[torch.Tensor], dilation, scale, tile_n, pad_hi) -> torch.Tensor:
+    # `out` None: allocated here, and then known to be a plain channels-last tensor. What a call costs on the host is of the
+    # size of a small convolution on the device, so every check below is made once and from plain ints.
     x, N, C, H, W, ldx = nhwc_view(x, "x")
     w = _krsc(w)
     K, Cw, R, S = w.shape
@@ -237,14 +248,19 @@ def conv_fused_into(x, w, bias, res, padding, stride, act: int, out: torch.Tenso
     ph_hi, pw_hi = (ph, pw) if pad_hi is None else _pair(pad_hi)
     P = (H + ph + ph_hi - dh * (R - 1) - 1) // sh + 1
     Q = (W + pw + pw_hi - dw * (S - 1) - 1) // sw + 1
-    out_v, No, Ko, Po, Qo, ldy = nhwc_view(out, "out")
-    if out_v is not out or (No, Ko, Po, Qo) != (N, K, P, Q):
-        raise FvmError(f"conv_fused_into: out must be a channels-last [N,K,P,Q]={N, K, P, Q} tensor or channel slice, "
-                       f"got {tuple(out.shape)} strides {out.stride()}")
+    fresh = out is None and K % 8 == 0
+    if out is None:
+        out = empty_nhwc(N, K, P, Q, x.device)
+    ldy = K
+    if not fresh:
+        out_v, No, Ko, Po, Qo, ldy = nhwc_view(out, "out")
+        if out_v is not out or (No, Ko, Po, Qo) != (N, K, P, Q):
+            raise FvmError(f"conv_fused_into: out must be a channels-last [N,K,P,Q]={N, K, P, Q} tensor or channel slice, "
+                           f"got {tuple(out.shape)} strides {out.stride()}")
     ldr = 0
     if res is not None:
         res, Nr, Kr, Pr, Qr, ldr = nhwc_view(res, "res")
-        if (Nr, Kr, Pr, Qr) != (N, K, P, Q):
+        if Nr != N or Kr != K or Pr != P or Qr != Q:
             raise FvmError("conv_fused: residual shape does not match the output")
     if bias is not None:
         _require_cuda_half(bias, "bias")
@@ -253,11 +269,11 @@ def conv_fused_into(x, w, bias, res, padding, stride, act: int, out: torch.Tenso
         if scale.dtype != torch.float32 or not scale.is_cuda:
             raise FvmError("conv_fused: scale must be an fp32 CUDA tensor")
         scale = scale.contiguous()
-    args = [x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(res), _ptr(scale), out.data_ptr(), N, H, W, C, K, R, S, ph, pw,
-            sh, sw, dh, dw, ldx, ldy, ldr, int(act)]
+    args = (x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(res), _ptr(scale), out.data_ptr(), N, H, W, C, K, R, S, ph, pw,
+            sh, sw, dh, dw, ldx, ldy, ldr, int(act))
     if _chain is not None and pad_hi is None and C >= 24:
         _chain.add(args, tile_n, (x, w, bias, res, scale, out))
-        return
+        return out
     L = lib()
     if pad_hi is not None:
         rc = L.fvm_conv2d_f16_pad(*args, int(tile_n), ph_hi, pw_hi, _stream())
@@ -265,23 +281,17 @@ def conv_fused_into(x, w, bias, res, padding, stride, act: int, out: torch.Tenso
         rc = L.fvm_conv2d_f16_tile(*args, int(tile_n), _stream())
     else:
         rc = L.fvm_conv2d_f16(*args, _stream())
-    _check(rc, "conv2d_f16")
+    if rc:
+        _check(rc, "conv2d_f16")
+    return out
 
 
 def conv_fused(x, w, bias=None, res=None, padding=(0, 0), stride=(1, 1), act: int = 0, cfg: int = -1,
                dilation=(1, 1), scale=None, tile_n: int = 0) -> torch.Tensor:
     """clf::conv_fused(x, w, bias?, res?, padding, stride, act, cfg=-1) -> Tensor (fused_conv.cu:298-302, schema :624).
     `cfg` (the reference's CUTLASS tile index) is accepted and ignored; `tile_n` forces this library's own N tile."""
-    N, C, H, W = x.shape
-    K, _, R, S = w.shape
-    ph, pw = _pair(padding)
-    sh, sw = _pair(stride)
-    dh, dw = _pair(dilation)
-    P = (H + 2 * ph - dh * (R - 1) - 1) // sh + 1
-    Q = (W + 2 * pw - dw * (S - 1) - 1) // sw + 1
-    out = empty_nhwc(N, K, P, Q, x.device)
-    conv_fused_into(x, w, bias, res, padding, stride, act, out, dilation=dilation, scale=scale, tile_n=tile_n)
-    return out
+    init(x.device)
+    return _conv(x, w, bias, res, padding, stride, act, None, dilation, scale, tile_n, None)
 
 
 def conv_fused_d(x, w, bias, res, padding, stride, dilation, act: int) -> torch.Tensor:
