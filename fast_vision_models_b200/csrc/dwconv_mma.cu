@@ -7,9 +7,11 @@
 // in two registers per lane, and each loaded input row feeds the 7 output rows it belongs to: 7 fp32 accumulator
 // fragments rotate through the registers. Per 128 outputs that is 7 matrix instructions and little more than one ldmatrix;
 // 7 of 16 products are useful. The fp16x2 FMA kernel (dw_tile_kernel) is bound by the FMA pipe and by reading every input
-// vector several times from shared memory; this one by the rate of mma.sync (about 5.5 cycles each per SM).
-// ConvNeXt-T layers, batch 64, us with the FMA kernel / this one (of HBM bandwidth): 56x56x96 62.7 / 39.2 (0.30),
-// 28x28x192 35.0 / 23.9, 14x14x384 29.2 / 15.5, 7x7x768 14.0 / 12.1; batch 8 at 56x56x96 12.1 / 9.0.
+// vector several times from shared memory; this one by the four barriers of a tile and its serial chains (with a predicate per matrix
+// instruction, 39 us for 56x56x96, the hmma pipe was busy 39 % of the time, the schedulers 43 %; three blocks per SM instead of
+// two need 80 registers a thread and gain nothing: 29.0 us).
+// ConvNeXt-T layers, batch 64, us with the FMA kernel / this one (share of HBM bandwidth): 56x56x96 62.7 / 27.9 (0.43),
+// 28x28x192 35.0 / 18.5 (0.32), 14x14x384 29.2 / 12.6, 7x7x768 14.0 / 9.3; batch 8 at 56x56x96 12.1 / 8.2.
 // With 3 or 5 taps the useful share is too small: 95x95x192 3x3 191 us against 128, 48x48x336 5x5 125 against 86 (tile kernel).
 //
 // The matrix unit wants one channel's columns side by side, NHWC has the channels side by side, so a block's input patch is
@@ -20,7 +22,7 @@
 //   C: output planes           -> B: [image][row][column][8 channels], stored by one TMA copy (clipped at the map's edges).
 // Blocks are persistent: a block keeps its 8 channels (a warp its channel, with the Toeplitz matrices in registers) and walks
 // tiles; the next patch is on its way to A while the present one is multiplied. Two blocks share an SM. Blocks of 8 channels
-// were faster than 16 and 32 (56x56x96, batch 64: 39 / 50 / 90 us): they allow the tallest segments, and a segment pays six
+// were faster than 16 and 32 (56x56x96, batch 64, with predicates: 39 / 50 / 90 us): they allow the tallest segments, and a segment pays six
 // rows of border.
 //
 // A column outside an output's window meets a zero of the Toeplitz matrix, which is harmless for finite values only. The
@@ -79,6 +81,9 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 
+struct TrueTag { static constexpr bool value = true; };
+struct FalseTag { static constexpr bool value = false; };
+
 // fp32 pair -> rounded fp16 pair -> activation (evaluated on the rounded sum, rounded again: as dw_tile_kernel does)
 template <int ACT>
 __device__ __forceinline__ uint32_t dm_finish(float lo, float hi, int act) {
@@ -113,7 +118,9 @@ __device__ __noinline__ void dw7_direct_part(const DmParams& p, const uint8_t* p
     }
 }
 
-template <int ACT>
+// ANYROWS: segments of any height; false: a multiple of 7 rows, so that the first and the last 7 input rows of a strip know at
+// compile time which products they have (no predicate per matrix instruction).
+template <int ACT, bool ANYROWS>
 __global__ void __launch_bounds__(DM_THREADS, 2)
 dw7_mma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
               const __half* __restrict__ w, const __half* __restrict__ bias, float* __restrict__ pool_partial,
@@ -234,39 +241,64 @@ dw7_mma_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 uint32_t dst = o0 + static_cast<uint32_t>(c * p.oplane + (lane & 15) * 16);
                 uint32_t nxt[4];
                 ldsm_x4(nxt, src);
+                auto emit = [&](const float (&d)[4], int row) {
+                    const uint32_t h0 = dm_finish<ACT>(d[0], d[1], p.act), h1 = dm_finish<ACT>(d[2], d[3], p.act);
+                    stsm_x2(dst, h0, h1);
+                    dst += 256;
+                    if (pool_partial) {
+                        const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&h0));
+                        const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
+                        if (row < rows_ok[0]) sum0 += (cols_ok[0] > 0 ? f0.x : 0.f) + (cols_ok[0] > 1 ? f0.y : 0.f);
+                        if (row < rows_ok[1]) sum1 += (cols_ok[1] > 0 ? f1.x : 0.f) + (cols_ok[1] > 1 ? f1.y : 0.f);
+                    }
+                };
                 // rotating accumulators: input row y belongs to output rows y - r, r = 0 .. S - 1; row y - r sits in slot
                 // (y - r) mod S; products for rows before the first or past the last are skipped.
-                for (int y0 = 0; y0 < rows; y0 += S) {
+                if constexpr (ANYROWS) {
+                    for (int y0 = 0; y0 < rows; y0 += S) {
 #pragma unroll
-                    for (int j = 0; j < S; ++j) {
-                        const int y = y0 + j;
-                        if (y < rows) {
-                            uint32_t a[4] = {nxt[0], nxt[1], nxt[2], nxt[3]};
-                            if (y + 1 < rows) src += row_bytes;
-                            ldsm_x4(nxt, src);                           // the next row under this row's products
+                        for (int j = 0; j < S; ++j) {
+                            const int y = y0 + j;
+                            if (y < rows) {
+                                uint32_t a[4] = {nxt[0], nxt[1], nxt[2], nxt[3]};
+                                if (y + 1 < rows) src += row_bytes;
+                                ldsm_x4(nxt, src);                       // the next row under this row's products
 #pragma unroll
-                            for (int r = 0; r < S; ++r) {
-                                float (&d)[4] = acc[(j - r + S) % S];
-                                if (y - r < p.rr) {
-                                    if (r == 0) mma_16816(d, a, bw[r][0], bw[r][1], bc, bc, bc, bc);
-                                    else if (j >= r || y0 > 0) mma_16816(d, a, bw[r][0], bw[r][1], d[0], d[1], d[2], d[3]);
+                                for (int r = 0; r < S; ++r) {
+                                    float (&d)[4] = acc[(j - r + S) % S];
+                                    if (y - r < p.rr) {
+                                        if (r == 0) mma_16816(d, a, bw[r][0], bw[r][1], bc, bc, bc, bc);
+                                        else if (j >= r || y0 > 0) mma_16816(d, a, bw[r][0], bw[r][1], d[0], d[1], d[2], d[3]);
+                                    }
                                 }
-                            }
-                            const int row = y - (S - 1);
-                            if (row >= 0) {
-                                const float (&d)[4] = acc[(j + 1) % S];
-                                const uint32_t h0 = dm_finish<ACT>(d[0], d[1], p.act), h1 = dm_finish<ACT>(d[2], d[3], p.act);
-                                stsm_x2(dst, h0, h1);
-                                dst += 256;
-                                if (pool_partial) {
-                                    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&h0));
-                                    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
-                                    if (row < rows_ok[0]) sum0 += (cols_ok[0] > 0 ? f0.x : 0.f) + (cols_ok[0] > 1 ? f0.y : 0.f);
-                                    if (row < rows_ok[1]) sum1 += (cols_ok[1] > 0 ? f1.x : 0.f) + (cols_ok[1] > 1 ? f1.y : 0.f);
-                                }
+                                if (y >= S - 1) emit(acc[(j + 1) % S], y - (S - 1));
                             }
                         }
                     }
+                } else {
+                    auto seven = [&](auto first_, auto last_, int y0) {
+                        constexpr bool FIRST = decltype(first_)::value, LAST = decltype(last_)::value;
+#pragma unroll
+                        for (int j = 0; j < (LAST ? S - 1 : S); ++j) {
+                            uint32_t a[4] = {nxt[0], nxt[1], nxt[2], nxt[3]};
+                            if (!LAST || j < S - 2) {
+                                src += row_bytes;
+                                ldsm_x4(nxt, src);                       // the next row under this row's products
+                            }
+#pragma unroll
+                            for (int r = 0; r < S; ++r) {
+                                float (&d)[4] = acc[(j - r + S) % S];
+                                if ((!FIRST || j >= r) && (!LAST || j < r)) {
+                                    if (r == 0) mma_16816(d, a, bw[r][0], bw[r][1], bc, bc, bc, bc);
+                                    else mma_16816(d, a, bw[r][0], bw[r][1], d[0], d[1], d[2], d[3]);
+                                }
+                            }
+                            if (!FIRST || j == S - 1) emit(acc[(j + 1) % S], y0 + j - (S - 1));
+                        }
+                    };
+                    seven(TrueTag{}, FalseTag{}, 0);
+                    for (int y0 = S; y0 < p.rr; y0 += S) seven(FalseTag{}, FalseTag{}, y0);
+                    seven(FalseTag{}, TrueTag{}, p.rr);
                 }
                 if (pool_partial) {
                     sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
@@ -339,7 +371,7 @@ struct DmPlan {
 };
 
 // Tile geometry: the candidate with the least modelled time, per round of the persistent blocks: the matrix instructions
-// (about 310 cycles per output row of a tile's 16 strips x 8 channels) and the copies in and out of the two blocks of an SM,
+// (about 310 cycles per output row of a tile's 16 strips x 8 channels, 200 without predicates) and the copies in and out of the two blocks of an SM,
 // or, for a block alone, its own plus the latency of its copies and barriers. Fitted to a sweep of all geometries for 18 maps
 // (batch 1 to 64); a grid that puts a second block on each SM starts later (8x14x14x384: 5.9 us with 96 blocks, 6.5 with 192).
 static bool dm_plan(int N, int H, int W, int C, int ph, int pw, int sms, DmPlan* out) {
@@ -386,10 +418,10 @@ static bool dm_plan(int N, int H, int W, int C, int ph, int pw, int sms, DmPlan*
                     const double rounds = static_cast<double>((tiles + per_vb - 1) / per_vb) * ((d.grid + slots - 1) / slots);
                     const double on_sm = d.grid > static_cast<unsigned>(sms) ? 2.0 : 1.0;
                     if (on_sm > 1.0) {
-                        const double busy = 310.0 * rr + 3.0 * p.groups + 700.0;
+                        const double busy = (rr % S ? 310.0 : 200.0) * rr + 3.0 * p.groups + 700.0;
                         d.cost = rounds * (2500.0 + busy > 2.0 * busy ? 2500.0 + busy : 2.0 * busy) + 4000.0;
                     } else {
-                        d.cost = rounds * (2500.0 + 230.0 * rr + 3.0 * p.groups);
+                        d.cost = rounds * (2500.0 + (rr % S ? 230.0 : 160.0) * rr + 3.0 * p.groups);
                     }
                     if (!any || d.cost < out->cost) {
                         *out = d;
@@ -417,8 +449,8 @@ static bool dm_plan_cached(int N, int H, int W, int C, int ph, int pw, DmPlan* o
     return e.ok;
 }
 
-// Every stride-1 7x7 layer: at the small end both kernels are bound by launch and latency (us, tile kernel / this one: one image
-// 56x56x96 4.7 / 4.7, 14x14x384 5.1 / 4.6; batch 32 at 7x7x768 8.2 / 8.3), above it this one is faster throughout.
+// Every stride-1 7x7 layer: also at the small end this one is faster (us, tile kernel / this one: one image 56x56x96 4.7 / 4.1,
+// 14x14x384 5.1 / 3.9; 20 images 9x9x768 9.7 / 8.2).
 bool dw_mma_runs(int N, int H, int W, int C, int ph, int pw) {
     DmPlan d;
     return dm_plan_cached(N, H, W, C, ph, pw, &d);
@@ -448,7 +480,9 @@ int dw_mma_launch(const void* x, const void* w, const void* bias, void* y, float
         const int rc = encode_tiled_f16(o ? &ty : &tx, o ? y : x, 4, dims, strides, box, false);
         if (rc != FVM_OK) return rc;
     }
-    auto kernel = act == 0 ? dw7_mma_kernel<0> : dw7_mma_kernel<-1>;
+    const bool any = p.rr % DM_S != 0;
+    auto kernel = act == 0 ? (any ? dw7_mma_kernel<0, true> : dw7_mma_kernel<0, false>)
+                           : (any ? dw7_mma_kernel<-1, true> : dw7_mma_kernel<-1, false>);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DM_SMEM_LIMIT) != cudaSuccess) return FVM_ERR_SETUP;
     return launch_pdl(kernel, dim3(d.grid), dim3(DM_THREADS), d.smem, stream, 1, tx, ty, static_cast<const __half*>(w),
                       static_cast<const __half*>(bias), pool_partial, p);
