@@ -1,5 +1,6 @@
 // Library state and the C-ABI entry points that are not tied to one kernel file.
 #include <atomic>
+#include <cstdlib>
 #include <mutex>
 
 #include "fvm_internal.h"
@@ -17,6 +18,11 @@ DeviceState* device_state() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return nullptr;
     DeviceState* st = &g_state[dev];
     return st->ready ? st : nullptr;
+}
+
+bool pdl_enabled() {
+    static const bool on = [] { const char* v = getenv("FVM_B200_PDL"); return !(v && v[0] == '0'); }();
+    return on;
 }
 
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }

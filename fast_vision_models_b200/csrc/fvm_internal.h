@@ -73,6 +73,7 @@ int conv_dual_launch(const void* x, const void* w1, const void* b1, const void* 
                      void* z, long long M, int C1, int K1, int K2, long long ldx, long long ldr, long long ldy, long long ldz,
                      int act1, int act2, cudaStream_t stream);
 
+bool pdl_enabled();      // FVM_B200_PDL=0: plain launches
 // Launch with programmatic stream serialization (the kernel calls pdl_wait before it touches activations) in clusters of
 // `cluster` blocks. Measured on B200 in a replayed graph: a plain launch adds about 1 us between two small kernels.
 template <typename... P, typename... A>
@@ -89,8 +90,9 @@ int launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStr
     attrs[1].val.clusterDim.x = static_cast<unsigned>(cluster);
     attrs[1].val.clusterDim.y = 1;
     attrs[1].val.clusterDim.z = 1;
-    cfg.attrs = attrs;
-    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    const bool pdl = pdl_enabled();
+    cfg.attrs = pdl ? attrs : attrs + 1;
+    cfg.numAttrs = (pdl ? 1u : 0u) + (cluster > 1 ? 1u : 0u);
     if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) {
         (void)cudaGetLastError();
         return FVM_ERR_LAUNCH;

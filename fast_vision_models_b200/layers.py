@@ -228,12 +228,16 @@ class FusedConv(nn.Module):
                 except ops.FvmError:
                     continue
             # Each timed launch sees the cache state it has inside a forward pass: weights, residual and output cold
-            # (a buffer larger than L2 is overwritten first), the input freshly written (as by the previous layer).
+            # (a buffer larger than L2 is overwritten first), the input freshly written (as by the previous layer). A network
+            # over one small image stays in the 126 MB L2 from one pass to the next: its weights are read back first.
+            warm = x.shape[0] == 1 and x.numel() + out.numel() <= 1 << 20
             flush = _l2_flush_buffer(x.device)
             for _round in range(4):
                 for c in times:
                     for _ in range(2):
                         flush.zero_()
+                        if warm:
+                            torch.sum(self.w, dtype=torch.float32)
                         x.mul_(1)           # exact identity: rewrites the input, which puts it back into L2
                         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                         e0.record()
@@ -243,8 +247,13 @@ class FusedConv(nn.Module):
                         e1.synchronize()
                         times[c] = min(times[c], e0.elapsed_time(e1))
             best_ms = times.get(0, float("inf"))
-            for c, ms in times.items():
-                if ms < best_ms * 0.97:      # a different tile must be clearly faster than the incumbent
+            in_clusters = lambda c: (c >> 28) & 3 == 3
+            for c, ms in sorted(times.items(), key=lambda t: in_clusters(t[0])):
+                # a different tile must be clearly faster than the incumbent; a split reduction over more than a few tiles
+                # more so, because a launch timed alone does not show the weights that the persistent kernels' deeper
+                # pipelines fetch under the preceding layer (3x3 256 -> 256 at 13x17, batch 13: alone about equal, in the
+                # network 14.7 against 12.1 us)
+                if ms < best_ms * (0.90 if in_clusters(c) and not in_clusters(best) and rows > 1024 else 0.97):
                     best, best_ms = c, ms
         self._tiles[key] = best
         TileCache.put(dev_idx, ckey, best)
