@@ -6,7 +6,11 @@
 // run of k-blocks (TMA -> tcgen05.mma -> fp32 accumulator in its own TMEM), then sends row slice o of its partial tile to
 // CTA o's shared memory (distributed shared memory, 16-byte stores), and after one cluster barrier every CTA adds the
 // `split` partial sums of its slice in rank order, applies bias / scale / residual / activation in fp32 and writes the
-// result with 16-byte stores. (One bulk copy per slice instead of the remote stores was 0.5 to 2 us slower per launch.) No scratch in global memory, no flags, the same order of additions on every run.
+// result with 16-byte stores. (One bulk copy per slice instead of the remote stores was 0.5 to 2 us slower per launch.)
+// No scratch in global memory, no flags, the same order of additions on every run. Graph of 20 launches, against the best
+// CTA-pair tile, us: 3x3 512 -> 512 at 7x7, one image 6.5 / 18.8; 3x3 256 -> 256 at 14x14, one image 5.4 / 11.1; 1x1
+// 2048 -> 512 at 7x7 4.9 / 9.4; classifier 2048 -> 1000 5.2 / 9.4; but 1x1 256 -> 1024 at 14x14 5.4 / 4.5 and the second of
+// these at batch 64 38 / 17: the per-layer timing decides.
 // The stages and the exchange buffer stay below half of an SM's shared memory where the pipeline allows it, so that the
 // next layer's CTAs (programmatic dependent launch) can already fetch their weights beside this layer's last tiles.
 #include <cuda.h>

@@ -148,8 +148,8 @@ int fvm_conv2d_f16_pad(const void* x, const void* w, const void* bias, const voi
 /* Depthwise RxS convolution -- replaces clf::dwconv (fused_conv.cu:418-502), clfr3::dwconv2 (r3.cu:335-454) and
  * segx::dwconv (segmentation/fast/seg_kernels.cu:124-158):
  *   y[n,p,q,c] = act( bias[c] + sum_{r,s} x[n, p*sh-ph+r*dh, q*sw-pw+s*dw, c] * w[r,s,c] )
- * Square 3/5/7-tap filters with stride 1 or 2 and no dilation use the arithmetic of dwconv2 (fp16x2 FMAs within a
- * kernel row, fp32 across rows); every other shape accumulates in fp32 throughout.
+ * Square 3/5-tap filters with stride 1 or 2, and 7-tap ones with stride 2, without dilation use the arithmetic of dwconv2
+ * (fp16x2 FMAs within a kernel row, fp32 across rows); every other shape accumulates in fp32 throughout.
  * Fused squeeze (cf. gconv2_pool, r3.cu:181-203): if pool_partial != NULL it receives fp32 partial sums of the
  * fp16-rounded outputs, laid out [N][slots][C] with slots = fvm_dwconv_pool_slots(...) for the same geometry; every
  * element is written (no zeroing needed) and the sums do not depend on scheduling (no atomics). The mean over the
